@@ -575,7 +575,7 @@ int pimc_d_dbeta(pimc_context *ctx, int action, int slice1, int slice2, int leve
     if (!ctx->lr_ready) return fail(ctx, PIMC_E_STATE, "pimc_set_longrange not called");
     if (level >= ctx->lr_levels) return fail(ctx, PIMC_E_ARG, "level beyond the long-range tables");
     const LRDesc lr = lr_desc(ctx);
-    CK(launch_rhok_full(ctx->stream, ctx->d_path[0], ctx->sys.N, ctx->sys.S, lr, ctx->d_rhok[0]));
+    CK(launch_rhok_full(ctx->stream, ctx->d_path[0], ctx->sys.N, ctx->sys.S, lr, ctx->sm_count, ctx->d_rhok[0]));
     double ksum = 0.0;
     if (pa_long_range(ctx)) {
       ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->d_out};
@@ -778,7 +778,7 @@ static int run_bisection(pimc_context *ctx, int n_blocks, pimc_move_record *devi
   a.wait_cap = ctx->bis.wait_cap;
   a.test_wait = ctx->bis.test_wait;
   if (a.use_lr && !ctx->rhok_valid) {  // PathClass::UpdateRho_ks() of the current OLD path
-    CK(launch_rhok_full(ctx->stream, ctx->d_path[0], ctx->sys.N, ctx->sys.S, lr_desc(ctx), ctx->d_rhok[0]));
+    CK(launch_rhok_full(ctx->stream, ctx->d_path[0], ctx->sys.N, ctx->sys.S, lr_desc(ctx), ctx->sm_count, ctx->d_rhok[0]));
     ctx->rhok_valid = true;
   }
   const int cl = ctx->bis.cluster_ctas, thr = ctx->bis.threads_per_cta;
@@ -1072,7 +1072,7 @@ static int yk_single(pimc_context *ctx, int copy, int slice1, int slice2, const 
 static int yk_sum(pimc_context *ctx, int slice1, int slice2, int table, double *out) {
   if (!ctx->yk_ready) return fail(ctx, PIMC_E_STATE, "pimc_davidlongrange_yk not called");
   const LRDesc lr = lr_desc(ctx);
-  CK(launch_rhok_full(ctx->stream, ctx->d_path[0], ctx->sys.N, ctx->sys.S, lr, ctx->d_rhok[0]));
+  CK(launch_rhok_full(ctx->stream, ctx->d_path[0], ctx->sys.N, ctx->sys.S, lr, ctx->sm_count, ctx->d_rhok[0]));
   ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->d_out};
   CK(launch_lr_sum(t, ctx->d_rhok[0], lr, ctx->d_yk + (size_t)table * ctx->num_k, slice1, slice2, 1, ctx->sm_count,
                    0.5));
@@ -1091,7 +1091,7 @@ int pimc_calc_rhok(pimc_context *ctx) {
   if (!ctx) return PIMC_E_ARG;
   if (ctx->num_k <= 0) return fail(ctx, PIMC_E_STATE, "pimc_setup_kvecs not called");
   CK(cudaSetDevice(ctx->device));
-  CK(launch_rhok_full(ctx->stream, ctx->d_path[0], ctx->sys.N, ctx->sys.S, lr_desc(ctx), ctx->d_rhok[0]));
+  CK(launch_rhok_full(ctx->stream, ctx->d_path[0], ctx->sys.N, ctx->sys.S, lr_desc(ctx), ctx->sm_count, ctx->d_rhok[0]));
   CK(cudaMemcpyAsync(ctx->d_rhok[1], ctx->d_rhok[0], (size_t)ctx->sys.S * ctx->num_k * sizeof(double2),
                      cudaMemcpyDeviceToDevice, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));

@@ -13,11 +13,16 @@
 // C_d(1) = (cos, sin)(kBox_d x_d), C_d(-n) = conj(C_d(n)), and a k-vector's
 // term is (C_0(kx) C_1(ky)) C_2(kz).  The tables of the particles a block
 // handles are built cooperatively in shared memory.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "action_kernels.cuh"
 #include "device_math.cuh"
 #include "longrange.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace pimc {
 
@@ -27,19 +32,21 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// Fills C[d][n + kmax_d] for one position into shared memory (called by
-// threads 0..2, one dimension each).
-__device__ __forceinline__ void fill_phase_table(const double *r, int d, const LRDesc &lr, double2 *C) {
+// Fills C[d][n + kmax_d] for one coordinate x of dimension d into shared
+// memory (one thread per dimension).
+__device__ __forceinline__ void fill_phase_table(double x, int d, const LRDesc &lr, double2 *C) {
   const int m = lr.kmax[d];
-  const double phi = r[d] * lr.kbox[d];
+  const double phi = x * lr.kbox[d];
   double s, c;
   sincos(phi, &s, &c);
   const double2 t = make_double2(c, s);
   double2 *Cd = C + lr.coff[d];
-  Cd[m] = make_double2(1.0, 0.0);
+  double2 w = make_double2(1.0, 0.0);  // the running power stays in registers: a shared-memory round trip a step costs more
+  Cd[m] = w;
   for (int n = 1; n <= m; n++) {
-    Cd[m + n] = cmul(t, Cd[m + n - 1]);
-    Cd[m - n] = make_double2(Cd[m + n].x, -Cd[m + n].y);
+    w = cmul(t, w);
+    Cd[m + n] = w;
+    Cd[m - n] = make_double2(w.x, -w.y);
   }
 }
 
@@ -50,35 +57,83 @@ __device__ __forceinline__ double2 k_term(const double2 *C, const LRDesc &lr, in
 
 constexpr int kMaxPhase = 3 * (2 * 64 + 1);  // kmax <= 64 per dimension
 
-// One block per slice: rho_k(slice) = sum over particles of the k terms.
-__global__ void __launch_bounds__(256) rhok_full_kernel(const double *__restrict__ path, int N, LRDesc lr,
+// rho_k(slice) = sum over particles of the k terms: one cluster of CL blocks
+// per slice, each block a contiguous share of the particles.  A block builds
+// the phase tables of up to `batch` particles at once (thread t: particle
+// t / 3, dimension t % 3), then every thread adds its k-vectors' terms of the
+// whole batch; at the end the cluster's partial sums are added in rank order
+// through distributed shared memory, so the result is reproducible.
+// What bounds it: the shared-memory reads of the phases (three 16-byte reads
+// per k-vector and particle against 10 FP64 operations; neighbouring threads
+// share kx and ky, so most are broadcasts) and, at few particles per block, the
+// latency of sincos and of the recurrence.  Measured against one block per
+// slice that builds one particle's table at a time between two barriers
+// (pimc_calc_rhok): N = 128, 65 slices, 510 k-vectors 142 -> 26 us (the kernel
+// 139 -> 15), N = 1024, 65 slices, 787 k-vectors 1397 -> 104 us, N = 4000, 3
+// slices, 230 k-vectors 3347 -> 48 us.
+__global__ void __launch_bounds__(256) rhok_full_kernel(const double *__restrict__ path, int N, LRDesc lr, int batch,
                                                         double2 *rhok) {
-  __shared__ double2 C[kMaxPhase];
-  const int slice = blockIdx.x;
+  extern __shared__ double2 sh2[];  // phase tables [batch][tab], then the partial sums [nk]
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), CL = (int)cluster.num_blocks();
+  const int slice = (int)blockIdx.x / CL;
+  const int tab = lr.coff[2] + 2 * lr.kmax[2] + 1;
+  const int per = (N + CL - 1) / CL, beg = min(N, rank * per), end = min(N, beg + per);
   double2 acc[4];
-  const int per = (lr.nk + blockDim.x - 1) / blockDim.x;  // <= 4 (nk <= 1024)
-  for (int j = 0; j < 4; j++) acc[j] = make_double2(0.0, 0.0);
-  for (int p = 0; p < N; p++) {
-    __syncthreads();
-    if (threadIdx.x < 3) {
-      const double *r = path + ((size_t)slice * N + p) * 3;
-      double rr[3] = {r[0], r[1], r[2]};
-      fill_phase_table(rr, threadIdx.x, lr, C);
+  int o0[4], o1[4], o2[4];  // this thread's k-vectors (nk <= 1024): offsets into a phase table
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    acc[j] = make_double2(0.0, 0.0);
+    const int k = threadIdx.x + j * blockDim.x;
+    const int3 ki = k < lr.nk ? lr.kidx[k] : make_int3(0, 0, 0);
+    o0[j] = lr.coff[0] + ki.x;
+    o1[j] = lr.coff[1] + ki.y;
+    o2[j] = lr.coff[2] + ki.z;
+  }
+  for (int p0 = beg; p0 < end; p0 += batch) {
+    const int np = min(batch, end - p0);
+    for (int t = threadIdx.x; t < 3 * np; t += blockDim.x) {
+      const int p = t / 3, d = t - 3 * p;
+      fill_phase_table(path[((size_t)slice * N + p0 + p) * 3 + d], d, lr, sh2 + (size_t)p * tab);
     }
     __syncthreads();
-    for (int j = 0; j < per; j++) {
-      const int k = threadIdx.x + j * blockDim.x;
-      if (k < lr.nk) {
-        const double2 t = k_term(C, lr, lr.kidx[k]);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if ((int)threadIdx.x + j * (int)blockDim.x >= lr.nk) break;
+#pragma unroll 2
+      for (int p = 0; p < np; p++) {
+        const double2 *C = sh2 + (size_t)p * tab;
+        const double2 t = cmul(cmul(C[o0[j]], C[o1[j]]), C[o2[j]]);
         acc[j].x += t.x;
         acc[j].y += t.y;
       }
     }
+    __syncthreads();
   }
-  for (int j = 0; j < per; j++) {
+  if (CL == 1) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int k = threadIdx.x + j * blockDim.x;
+      if (k < lr.nk) rhok[(size_t)slice * lr.nk + k] = acc[j];
+    }
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
     const int k = threadIdx.x + j * blockDim.x;
-    if (k < lr.nk) rhok[(size_t)slice * lr.nk + k] = acc[j];
+    if (k < lr.nk) sh2[k] = acc[j];
   }
+  cluster.sync();
+  for (int k = rank * (int)blockDim.x + (int)threadIdx.x; k < lr.nk; k += CL * (int)blockDim.x) {
+    double2 v = make_double2(0.0, 0.0);
+    for (int r = 0; r < CL; r++) {
+      const double2 w = cluster.map_shared_rank(sh2, r)[k];
+      v.x += w.x;
+      v.y += w.y;
+    }
+    rhok[(size_t)slice * lr.nk + k] = v;
+  }
+  cluster.sync();  // no block leaves while a peer reads its sums
 }
 
 // One block per updated slice (slice1 + b*skip): NEW = OLD, then per active
@@ -99,13 +154,9 @@ __global__ void __launch_bounds__(256) rhok_update_kernel(const double *__restri
     __syncthreads();
     const int p = act.p[pi];
     if (threadIdx.x < 3) {
-      const double *r = path_new + ((size_t)slice * N + p) * 3;
-      double rr[3] = {r[0], r[1], r[2]};
-      fill_phase_table(rr, threadIdx.x, lr, Cn);
+      fill_phase_table(path_new[((size_t)slice * N + p) * 3 + threadIdx.x], threadIdx.x, lr, Cn);
     } else if (threadIdx.x >= 32 && threadIdx.x < 35) {
-      const double *r = path_old + ((size_t)slice * N + p) * 3;
-      double rr[3] = {r[0], r[1], r[2]};
-      fill_phase_table(rr, threadIdx.x - 32, lr, Co);
+      fill_phase_table(path_old[((size_t)slice * N + p) * 3 + threadIdx.x - 32], threadIdx.x - 32, lr, Co);
     }
     __syncthreads();
     for (int j = 0; j < per; j++) {
@@ -189,9 +240,30 @@ __global__ void rhok_copy_kernel(const double2 *__restrict__ src, double2 *dst, 
 
 }  // namespace
 
-cudaError_t launch_rhok_full(cudaStream_t st, const double *path, int N, int S, const LRDesc &lr, double2 *rhok) {
-  rhok_full_kernel<<<S, 256, 0, st>>>(path, N, lr, rhok);
-  return cudaGetLastError();
+// Blocks per slice: doubled until about four blocks come to every SM (their
+// sincos and table latencies overlap), while each keeps eight particles or
+// more; one block per slice where the slices alone do that.
+cudaError_t launch_rhok_full(cudaStream_t st, const double *path, int N, int S, const LRDesc &lr, int sm_count,
+                             double2 *rhok) {
+  int cl = 1;
+  while (cl < 8 && S * cl < 4 * sm_count && N >= 16 * cl) cl *= 2;
+  const int tab = lr.coff[2] + 2 * lr.kmax[2] + 1;
+  const int share = (N + cl - 1) / cl;
+  // tables of as many particles as 45 KB hold (kmax <= 64: 7 or more), 85 at most (a thread per particle and dimension)
+  const int batch = std::min(share, std::max(1, std::min(85, 45 * 1024 / (tab * (int)sizeof(double2)))));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(S * cl, 1, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)std::max(batch * tab, lr.nk) * sizeof(double2);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cl;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, rhok_full_kernel, path, N, lr, batch, rhok);
 }
 
 cudaError_t launch_rhok_update(cudaStream_t st, const double *path_old, const double *path_new, int N,

@@ -18,7 +18,8 @@ struct LRDesc {
   const int3 *kidx;
 };
 
-cudaError_t launch_rhok_full(cudaStream_t st, const double *path, int N, int S, const LRDesc &lr, double2 *rhok);
+cudaError_t launch_rhok_full(cudaStream_t st, const double *path, int N, int S, const LRDesc &lr, int sm_count,
+                             double2 *rhok);
 cudaError_t launch_rhok_update(cudaStream_t st, const double *path_old, const double *path_new, int N,
                                const LRDesc &lr, const ActiveList &act, int slice1, int slice2, int skip,
                                const double2 *rho_old, double2 *rho_new);
