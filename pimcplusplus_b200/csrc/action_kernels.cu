@@ -105,36 +105,7 @@ __device__ __forceinline__ void tri_decode(long long k, int &p1, int &p2) {
   p2 = (int)(k - a * (a - 1) / 2);
 }
 
-// ShortRangeClass::d_dBeta (ShortRangeClass.cc:316-355), FP64.
-template <int KIND>
-__global__ void __launch_bounds__(256) sr_dbeta_kernel(const double *__restrict__ path, DevSystem sys, DevPA pa,
-                                                       int slice1, int skip, int nlinks, int level, double *partials,
-                                                       unsigned int *counter, double *out) {
-  __shared__ double sh[32];
-  const int N = sys.N;
-  const long long npairs = (long long)N * (N - 1) / 2;
-  const long long total = npairs * nlinks;
-  double acc = 0.0;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int link = (int)(idx / npairs);
-    int p1, p2;
-    tri_decode(idx - (long long)link * npairs, p1, p2);
-    const int slice = slice1 + link * skip;
-    double a1[3], a2[3], b1[3], b2[3], dA[3], dB[3];
-    load3(path + ((size_t)slice * N + p1) * 3, a1);
-    load3(path + ((size_t)slice * N + p2) * 3, a2);
-    load3(path + ((size_t)(slice + skip) * N + p1) * 3, b1);
-    load3(path + ((size_t)(slice + skip) * N + p2) * 3, b2);
-    dist_disp(a1, a2, b1, b2, sys, dA, dB);
-    LinkGeom<double> g = link_geom<double>(dA, dB);
-    acc += pa_dU<KIND>(pa, g, level);
-  }
-  double r = block_sum(acc, sh);
-  finish_sum(r, partials, counter, out, sh);
-}
-
-// ---- observables: ShortRangePotClass::V and PairCorrelationClass::Accumulate ----
+// ---- observables: PairCorrelationClass::Accumulate ----
 // PathClass::DistDisp one-slice form (PathClass.h:637-660): minimum image by
 // nearbyint(disp / L), then |disp|.
 __device__ __forceinline__ double dist_one_slice(const double a[3], const double b[3], const DevSystem &s) {
@@ -149,79 +120,36 @@ __device__ __forceinline__ double dist_one_slice(const double a[3], const double
   return sqrt(d2);
 }
 
-// V(r) of the pair action: DavidPAClass::V (DavidPAClass.cc:104-113), column 0
-// of the first tau table with r clamped to the grid; PAtricubicFit's
-// potential spline (PAFitBase.h:82).
-template <int KIND>
-__device__ __forceinline__ double pa_V(const DevPA &pa, double r) {
-  if (KIND == PA_DAVID) {
-    const DDavid<double> &d = pa.d64;
-    const DGrid<double> &g = d.grid;
-    if (r > g.end) r = g.end;
-    if (r < g.start) r = g.start;
-    return spline_col(g, d.uy, d.ud2, d.ncols, 0, r);
-  }
-  if (KIND == PA_COULOMB) {
-    // CoulombPot V = Z1Z2 / r, less Vlong with the long-range breakup
-    // (ShortRangePotClass.cc:41-43); for the classical Coulomb action the V
-    // breakup fits the same X_k as the dU one, so Vlong is dUlong.
-    const DCoulomb<double> &c = pa.c64;
-    double v = c.z1z2 / r;
-    if (c.long_range) v -= quintic_at(c, c.dulong, r);
-    return v;
-  }
-  return pot_V(pa.t64, r);
-}
-
-// One pass over slices [0, S-1] x pairs p2 < p1 of the OLD path.
-//  DO_V: sum over slices of factor * sum_pairs V(r), factor 1/2 at the end
-//        slices (ActionsClass.cc:852-857 with ShortRangePotClass.cc:28-47).
-//  DO_G: histogram of the pair distances at slices [0, S-2] below the grid
-//        end, bin (int)nearbyint((r - start) * deltainv - 0.5)
-//        (ObservableCorrelation.cc:191-207, Grid.h:81-84); bins counted per
-//        block in shared memory, then added to the 64-bit histogram.
-template <int KIND, bool DO_V, bool DO_G>
-__global__ void __launch_bounds__(256) pair_obs_kernel(const double *__restrict__ path, DevSystem sys, DevPA pa,
-                                                       GofrGrid gg, unsigned long long *hist, double *partials,
-                                                       unsigned int *counter, double *out) {
+// The g(r) histogram: one pass over slices [0, S-2] x pairs p2 < p1 of the OLD
+// path, pair distances below the grid end in bin
+// (int)nearbyint((r - start) * deltainv - 0.5) (ObservableCorrelation.cc:
+// 191-207, Grid.h:81-84); bins counted per block in shared memory, then added
+// to the 64-bit histogram.
+__global__ void __launch_bounds__(256) gofr_kernel(const double *__restrict__ path, DevSystem sys, GofrGrid gg,
+                                                   unsigned long long *hist) {
   extern __shared__ unsigned int s_hist[];
-  __shared__ double sh[32];
   const int N = sys.N, S = sys.S;
   const long long npairs = (long long)N * (N - 1) / 2;
-  const long long total = npairs * S;
-  if (DO_G) {
-    for (int i = threadIdx.x; i < gg.nbins; i += blockDim.x) s_hist[i] = 0u;
-    __syncthreads();
-  }
-  double acc = 0.0;
+  const long long total = npairs * (S - 1);
+  for (int i = threadIdx.x; i < gg.nbins; i += blockDim.x) s_hist[i] = 0u;
+  __syncthreads();
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     const int slice = (int)(idx / npairs);
     int p1, p2;
     tri_decode(idx - (long long)slice * npairs, p1, p2);
-    if (!DO_V && slice == S - 1) continue;
     double a[3], b[3];
     load3(path + ((size_t)slice * N + p1) * 3, a);
     load3(path + ((size_t)slice * N + p2) * 3, b);
     const double dist = dist_one_slice(a, b, sys);
-    if (DO_V) {
-      const double f = (slice == 0 || slice == S - 1) ? 0.5 : 1.0;
-      acc += f * pa_V<KIND>(pa, dist);
-    }
-    if (DO_G && slice < S - 1 && dist < gg.end) {
+    if (dist < gg.end) {
       const int bin = (int)rint(rsub(rmul(rsub(dist, gg.start), gg.deltainv), 0.5));
       if (bin >= 0 && bin < gg.nbins) atomicAdd(&s_hist[bin], 1u);
     }
   }
-  if (DO_G) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < gg.nbins; i += blockDim.x)
-      if (s_hist[i]) atomicAdd(&hist[i], (unsigned long long)s_hist[i]);
-  }
-  if (DO_V) {
-    const double r = block_sum(acc, sh);
-    finish_sum(r, partials, counter, out, sh);
-  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < gg.nbins; i += blockDim.x)
+    if (s_hist[i]) atomicAdd(&hist[i], (unsigned long long)s_hist[i]);
 }
 
 __device__ __forceinline__ void velocity(const double *__restrict__ path, int N, int sa, int sb, int p,
@@ -360,22 +288,6 @@ cudaError_t launch_sr_single(const ReduceTarget &t, const double *path, const De
   return cudaGetLastError();
 }
 
-cudaError_t launch_sr_dbeta(const ReduceTarget &t, const double *path, const DevSystem &sys, const DevPA &pa,
-                            int slice1, int skip, int nlinks, int level, int sm_count) {
-  long long items = (long long)sys.N * (sys.N - 1) / 2 * nlinks;
-  int blocks = grid_for(items, 256, sm_count);
-  if (pa.kind == PA_DAVID)
-    sr_dbeta_kernel<PA_DAVID><<<blocks, 256, 0, t.stream>>>(path, sys, pa, slice1, skip, nlinks, level, t.partials,
-                                                            t.counter, t.out);
-  else if (pa.kind == PA_COULOMB)
-    sr_dbeta_kernel<PA_COULOMB><<<blocks, 256, 0, t.stream>>>(path, sys, pa, slice1, skip, nlinks, level, t.partials,
-                                                              t.counter, t.out);
-  else
-    sr_dbeta_kernel<PA_TRICUBIC><<<blocks, 256, 0, t.stream>>>(path, sys, pa, slice1, skip, nlinks, level, t.partials,
-                                                               t.counter, t.out);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_kin_single(const ReduceTarget &t, const double *path, const DevSystem &sys, const ActiveList &act,
                               int slice1, int skip, int nlinks, int level, int sm_count) {
   int blocks = grid_for((long long)act.n * nlinks, 256, sm_count);
@@ -392,40 +304,11 @@ cudaError_t launch_kin_dbeta(const ReduceTarget &t, const double *path, const De
   return cudaGetLastError();
 }
 
-cudaError_t launch_pair_obs(const ReduceTarget &t, const double *path, const DevSystem &sys, const DevPA &pa,
-                            bool do_v, const GofrGrid *gg, unsigned long long *hist, int sm_count) {
-  const long long items = (long long)sys.N * (sys.N - 1) / 2 * sys.S;
+cudaError_t launch_gofr(cudaStream_t st, const double *path, const DevSystem &sys, const GofrGrid &gg,
+                        unsigned long long *hist, int sm_count) {
+  const long long items = (long long)sys.N * (sys.N - 1) / 2 * (sys.S - 1);
   const int blocks = grid_for(items, 256, sm_count);
-  const size_t dyn = gg ? (size_t)gg->nbins * sizeof(unsigned int) : 0;
-  const GofrGrid g0 = gg ? *gg : GofrGrid{0.0, 0.0, 0.0, 0};
-  const bool dav = pa.kind == PA_DAVID;
-  if (do_v && pa.kind == PA_COULOMB) {
-    if (gg)
-      pair_obs_kernel<PA_COULOMB, true, true><<<blocks, 256, dyn, t.stream>>>(path, sys, pa, g0, hist, t.partials,
-                                                                              t.counter, t.out);
-    else
-      pair_obs_kernel<PA_COULOMB, true, false><<<blocks, 256, 0, t.stream>>>(path, sys, pa, g0, hist, t.partials,
-                                                                             t.counter, t.out);
-  } else if (do_v && gg) {
-    if (dav)
-      pair_obs_kernel<PA_DAVID, true, true><<<blocks, 256, dyn, t.stream>>>(path, sys, pa, g0, hist, t.partials,
-                                                                            t.counter, t.out);
-    else
-      pair_obs_kernel<PA_TRICUBIC, true, true><<<blocks, 256, dyn, t.stream>>>(path, sys, pa, g0, hist, t.partials,
-                                                                               t.counter, t.out);
-  } else if (do_v) {
-    if (dav)
-      pair_obs_kernel<PA_DAVID, true, false><<<blocks, 256, 0, t.stream>>>(path, sys, pa, g0, hist, t.partials,
-                                                                           t.counter, t.out);
-    else
-      pair_obs_kernel<PA_TRICUBIC, true, false><<<blocks, 256, 0, t.stream>>>(path, sys, pa, g0, hist, t.partials,
-                                                                              t.counter, t.out);
-  } else if (gg) {
-    pair_obs_kernel<PA_DAVID, false, true><<<blocks, 256, dyn, t.stream>>>(path, sys, pa, g0, hist, t.partials,
-                                                                          t.counter, t.out);
-  } else {
-    return cudaErrorInvalidValue;
-  }
+  gofr_kernel<<<blocks, 256, (size_t)gg.nbins * sizeof(unsigned int), st>>>(path, sys, gg, hist);
   return cudaGetLastError();
 }
 

@@ -93,7 +93,17 @@ int upload_david(pimc_context *ctx, const DavidTables &t, DDavid<R> &d) {
       diag[((size_t)lev * d.diag_stride + i) * 2] = (R)t.uy[src];
       diag[((size_t)lev * d.diag_stride + i) * 2 + 1] = (R)t.ud2[src];
     }
-  return upload(ctx, diag.data(), diag.size(), &d.diag);
+  if ((rc = upload(ctx, diag.data(), diag.size(), &d.diag))) return rc;
+  d.est = nullptr;
+  if (std::is_same<R, float>::value) return PIMC_OK;
+  std::vector<R> est((size_t)t.num_tau * np * 4);
+  for (size_t i = 0; i < (size_t)t.num_tau * np; i++) {
+    est[4 * i] = (R)t.uy[i * t.ncols];
+    est[4 * i + 1] = (R)t.ud2[i * t.ncols];
+    est[4 * i + 2] = (R)t.duy[i * t.ncols + 1];
+    est[4 * i + 3] = (R)t.dud2[i * t.ncols + 1];
+  }
+  return upload(ctx, est.data(), est.size(), &d.est);
 }
 
 int check_pair(pimc_context *ctx, int sp1, int sp2) {
@@ -240,6 +250,7 @@ int pimc_create(const pimc_system_desc *d, pimc_context **out) {
   if (e == cudaSuccess) e = cudaMemset(ctx->d_counter, 0, sizeof(unsigned int));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_out, 4 * sizeof(double));
   if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_out, 4 * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_bounds, pair_path_bounds_bytes(s.N, s.S));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_chain, kMaxChainStates * sizeof(ChainState));
   if (e == cudaSuccess) e = cudaMemset(ctx->d_chain, 0, kMaxChainStates * sizeof(ChainState));
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, d->device);
@@ -262,6 +273,7 @@ int pimc_destroy(pimc_context *ctx) {
   cudaFree(ctx->d_partials);
   cudaFree(ctx->d_counter);
   cudaFree(ctx->d_out);
+  cudaFree(ctx->d_bounds);
   if (ctx->h_out) cudaFreeHost(ctx->h_out);
   cudaFree(ctx->d_chain);
   cudaFree(ctx->d_trace);
@@ -601,7 +613,8 @@ int pimc_d_dbeta(pimc_context *ctx, int action, int slice1, int slice2, int leve
     case PIMC_ACTION_SHORTRANGE:
       if (ctx->pa.kind == PA_NONE) return fail(ctx, PIMC_E_STATE, "no pair action set");
       if (int rc2 = pa_levels_ok(ctx, level + 1)) return rc2;
-      CK(launch_sr_dbeta(t, path, ctx->sys, ctx->pa, slice1, skip, nlinks, level, ctx->sm_count));
+      CK(launch_pair_path(t, path, ctx->sys, ctx->pa, slice1, skip, nlinks, level, false, ctx->d_bounds,
+                          ctx->sm_count));
       break;
     case PIMC_ACTION_KINETIC:
       CK(launch_kin_dbeta(t, path, ctx->sys, slice1, skip, nlinks, level, ctx->sm_count));
@@ -1128,16 +1141,34 @@ int pimc_energy(pimc_context *ctx, pimc_energy_terms *out) {
   if (ctx->pa.kind == PA_NONE) return fail(ctx, PIMC_E_STATE, "no pair action set");
   CK(cudaSetDevice(ctx->device));
   const int M = ctx->sys.S - 1;
-  pimc_energy_terms e = {};
-  // ActionsClass::Energy (ActionsClass.cc:812-871) on the OLD path
-  int rc = pimc_d_dbeta(ctx, PIMC_ACTION_KINETIC, 0, M, 0, &e.kinetic);
-  if (!rc) rc = pimc_d_dbeta(ctx, PIMC_ACTION_SHORTRANGE, 0, M, 0, &e.du_short);
-  if (!rc && ctx->lr_ready) rc = pimc_d_dbeta(ctx, PIMC_ACTION_LONGRANGE, 0, M, 0, &e.du_long);
-  if (rc) return rc;
+  // ActionsClass::Energy (ActionsClass.cc:812-871) on the OLD path: the
+  // kinetic, short-range (with V) and long-range sums are enqueued one after
+  // another, each into its own scalar, and read back together.
+  if (int rc = pa_levels_ok(ctx, 1)) return rc;
+  const double *path = ctx->d_path[PIMC_OLD];
   ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->d_out};
-  CK(launch_pair_obs(t, ctx->d_path[PIMC_OLD], ctx->sys, ctx->pa, true, nullptr, nullptr, ctx->sm_count));
-  rc = finish_scalar(ctx, &e.v_short);
-  if (rc) return rc;
+  CK(launch_kin_dbeta(t, path, ctx->sys, 0, 1, M, 0, ctx->sm_count));
+  t.out = ctx->d_out + 1;
+  CK(launch_pair_path(t, path, ctx->sys, ctx->pa, 0, 1, M, 0, true, ctx->d_bounds, ctx->sm_count));
+  int n = 3;
+  if (ctx->lr_ready) {  // LongRangeClass::d_dBeta: rho_k of the OLD copy recomputed
+    const LRDesc lr = lr_desc(ctx);
+    CK(launch_rhok_full(ctx->stream, path, ctx->sys.N, ctx->sys.S, lr, ctx->sm_count, ctx->d_rhok[0]));
+    if (pa_long_range(ctx)) {
+      t.out = ctx->d_out + 3;
+      CK(launch_lr_sum(t, ctx->d_rhok[0], lr, ctx->d_dulong_k, 0, M, 1, ctx->sm_count));
+      n = 4;
+    }
+  }
+  CK(cudaMemcpyAsync(ctx->h_out, ctx->d_out, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  for (int i = 0; i < n; i++)
+    if (!std::isfinite(ctx->h_out[i])) return fail(ctx, PIMC_E_NAN, "non-finite action");
+  pimc_energy_terms e = {};
+  e.kinetic = ctx->h_out[0];
+  e.du_short = ctx->h_out[1];
+  e.v_short = ctx->h_out[2];
+  if (ctx->lr_ready) e.du_long = (n == 4 ? ctx->h_out[3] : 0.0) + lr_constant(ctx, 0, M, 0, true);
   e.v_long = 0.0;
   // EnergyClass::Accumulate's sample (ObservableEnergy.cc:45-73): per slice
   e.total = (e.kinetic + e.du_short + e.du_long) / (double)M;
@@ -1170,8 +1201,7 @@ int pimc_gofr_accumulate(pimc_context *ctx) {
   if (!ctx->d_gofr) return fail(ctx, PIMC_E_STATE, "pimc_gofr_setup not called");
   CK(cudaSetDevice(ctx->device));
   GofrGrid g{ctx->gofr_start, ctx->gofr_end, ctx->gofr_deltainv, ctx->gofr_points - 1};
-  ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->d_out};
-  CK(launch_pair_obs(t, ctx->d_path[PIMC_OLD], ctx->sys, ctx->pa, false, &g, ctx->d_gofr, ctx->sm_count));
+  CK(launch_gofr(ctx->stream, ctx->d_path[PIMC_OLD], ctx->sys, g, ctx->d_gofr, ctx->sm_count));
   ctx->gofr_counts++;
   return PIMC_OK;
 }

@@ -187,49 +187,6 @@ __device__ __forceinline__ R david_U(const DDavid<R> &d, const typename Pair2<R>
   return U;
 }
 
-// ---- DavidPAClass::calcUsqz, dU output (DavidPAClass.cc:291-463) ----
-template <typename R>
-__device__ __forceinline__ R david_dU(const DDavid<R> &d, R s2, R q, R z, int level) {
-  level = level + d.tau_pos;
-  const DGrid<R> &g = d.grid;
-  const R *uy = d.uy + (size_t)level * g.n * d.ncols;
-  const R *ud2 = d.ud2 + (size_t)level * g.n * d.ncols;
-  const R *dy = d.duy + (size_t)level * g.n * d.ncols;
-  const R *dd2 = d.dud2 + (size_t)level * g.n * d.ncols;
-  R rmin = g.start;
-  R r = q + R(0.5) * z;
-  R rprime = q - R(0.5) * z;
-  if (r > g.end) r = g.end;
-  if (rprime > g.end) rprime = g.end;
-  if (rprime < rmin) rprime = rmin;
-  if (r < rmin) r = rmin;
-  R V = R(0.5) * (spline_col(g, uy, ud2, d.ncols, 0, r) + spline_col(g, uy, ud2, d.ncols, 0, rprime));
-  R dU = R(0.5) * (spline_col(g, dy, dd2, d.ncols, 1, r) + spline_col(g, dy, dd2, d.ncols, 1, rprime));
-  dU += V;
-  if (d.num_terms > 0 && s2 > R(0) && q < g.end) {
-    const R s = sqrt_r(s2);
-    SplineCell<R> c = spline_cell(g, q);
-    R zsquared = z * z;
-    R ssquared = s * s;
-    R ssquaredinverse = R(1.0) / ssquared;
-    R Sto2k = ssquared;
-    for (int k = 1; k <= d.num_terms; k++) {
-      R Zto2j = 1;
-      R currS = Sto2k;
-      for (int j = 0; j <= k; j++) {
-        int col = k * (k + 1) / 2 + j + 1;
-        R dUcof = spline_apply(c, __ldg(&dy[c.low * d.ncols + col]), __ldg(&dy[c.hi * d.ncols + col]),
-                               __ldg(&dd2[c.low * d.ncols + col]), __ldg(&dd2[c.hi * d.ncols + col]));
-        dU += dUcof * Zto2j * currS;
-        Zto2j *= zsquared;
-        currS = currS * ssquaredinverse;
-      }
-      Sto2k = Sto2k * ssquared;
-    }
-  }
-  return dU;
-}
-
 // ---- MyTricubicSpline::operator() (MyTricubicSpline.h:197-334) ----
 // Hermite basis p1, p2, q1, q2 (MyTricubicSpline.h:38-45).
 template <typename R>
@@ -317,11 +274,11 @@ __device__ __forceinline__ R pot_V(const DTricubic<R> &t, R r) {
   return r <= t.pot_grid.end ? v : R(0);
 }
 
-// ---- PAtricubicFitClass::U / dU (PAtricubicFit.cc:659-721) ----
+// ---- PAtricubicFitClass::U (PAtricubicFit.cc:659-721) ----
 // Inside the fitted region (q <= qmax, z < 2q, s < 2q) the tricubic spline at
 // (q, z/2q, (s-z)/(2q-z)) (at (0,0,0) when q == 0); outside it the primitive
-// action 1/2 beta_l (V(r) + V(r')) (dU: 1/2 (V(r) + V(r'))).
-template <typename R, bool DERIV>
+// action 1/2 beta_l (V(r) + V(r')).
+template <typename R>
 __device__ __forceinline__ R tricubic_pa(const DTricubic<R> &t, R q, R z, R s2, int level, int part = 0,
                                          int nparts = 1) {
   const DGrid<R> &qg = t.qg, &yg = t.yg, &tg = t.tg;
@@ -334,16 +291,13 @@ __device__ __forceinline__ R tricubic_pa(const DTricubic<R> &t, R q, R z, R s2, 
   const R xq = nonzero ? q : R(0);
   const R xy = nonzero ? z / zmax : R(0);
   const R xt = nonzero ? (s - z) / (smax - z) : R(0);
-  const R *F = (DERIV ? t.dU : t.U) + (size_t)level * t.nq * t.ny * t.nt * 8;
+  const R *F = t.U + (size_t)level * t.nq * t.ny * t.nt * 8;
   const int k0 = (4 * part) / nparts, k1 = (4 * (part + 1)) / nparts;
   const R r = q + R(0.5) * z;
   const R rp = q - R(0.5) * z;
-  R beta = R(0.5);
-  if (!DERIV) {
-    beta = t.smallest_beta;
-    for (int i = 0; i < level; i++) beta *= R(2.0);
-    beta = R(0.5) * beta;
-  }
+  R beta = t.smallest_beta;
+  for (int i = 0; i < level; i++) beta *= R(2.0);
+  beta = R(0.5) * beta;
   if (nparts == 1) {
     // One lane, one term: a lane inside the fit gathers its cell, a lane
     // outside reads the two potential splines; in a warp with both, each
@@ -449,16 +403,6 @@ __device__ __forceinline__ R coulomb_U(const DCoulomb<R> &c, const LinkGeom<R> &
   }
   return U;
 }
-// PAclassicalFitClass::dU with dUlong taken out (ShortRangeClass.cc:282-286).
-__device__ __forceinline__ double coulomb_dU(const DCoulomb<double> &c, const LinkGeom<double> &g, int level) {
-  double dU = c.z1z2 / g.q;
-  if (c.long_range) {
-    const double *tab = c.dulong + (size_t)level * c.np * 6;
-    dU -= 0.5 * (quintic_at(c, tab, g.rmag) + quintic_at(c, tab, g.rpmag));
-  }
-  return dU;
-}
-
 template <typename R, int KIND>
 __device__ __forceinline__ R pa_U(const DevPA &pa, const typename Pair2<R>::T *diag, const LinkGeom<R> &g,
                                   int level);
@@ -486,13 +430,13 @@ template <>
 __device__ __forceinline__ double pa_U<double, PA_TRICUBIC>(const DevPA &pa, const double2 *,
                                                             const LinkGeom<double> &g, int level) {
   const DTricubic<double> &t = pa.t64;
-  return tricubic_pa<double, false>(t, g.q, g.z, g.s2, level);
+  return tricubic_pa<double>(t, g.q, g.z, g.s2, level);
 }
 template <>
 __device__ __forceinline__ float pa_U<float, PA_TRICUBIC>(const DevPA &pa, const float2 *,
                                                           const LinkGeom<float> &g, int level) {
   const DTricubic<float> &t = pa.t32;
-  return tricubic_pa<float, false>(t, g.q, g.z, g.s2, level);
+  return tricubic_pa<float>(t, g.q, g.z, g.s2, level);
 }
 
 // Part `part` of `nparts` of U for a team of lanes sharing one evaluation;
@@ -500,7 +444,7 @@ __device__ __forceinline__ float pa_U<float, PA_TRICUBIC>(const DevPA &pa, const
 template <typename R, int KIND>
 __device__ __forceinline__ R pa_U_part(const DevPA &pa, const typename Pair2<R>::T *diag, const LinkGeom<R> &g,
                                        int level, int part, int nparts) {
-  if (KIND == PA_TRICUBIC) return tricubic_pa<R, false>(tricubic_of<R>(pa), g.q, g.z, g.s2, level, part, nparts);
+  if (KIND == PA_TRICUBIC) return tricubic_pa<R>(tricubic_of<R>(pa), g.q, g.z, g.s2, level, part, nparts);
   return part == 0 ? pa_U<R, KIND>(pa, diag, g, level) : R(0);
 }
 
@@ -841,23 +785,6 @@ __device__ __forceinline__ void two_sum_add(double &s, float &c, double x) {
   const double bp = t - s;
   c += (float)((s - (t - bp)) + (x - bp));
   s = t;
-}
-
-// dU (energy estimator), FP64 only.
-template <int KIND>
-__device__ __forceinline__ double pa_dU(const DevPA &pa, const LinkGeom<double> &g, int level);
-template <>
-__device__ __forceinline__ double pa_dU<PA_DAVID>(const DevPA &pa, const LinkGeom<double> &g, int level) {
-  return david_dU<double>(pa.d64, g.s2, g.q, g.z, level);
-}
-template <>
-__device__ __forceinline__ double pa_dU<PA_COULOMB>(const DevPA &pa, const LinkGeom<double> &g, int level) {
-  return coulomb_dU(pa.c64, g, level);
-}
-template <>
-__device__ __forceinline__ double pa_dU<PA_TRICUBIC>(const DevPA &pa, const LinkGeom<double> &g, int level) {
-  const DTricubic<double> &t = pa.t64;
-  return tricubic_pa<double, true>(t, g.q, g.z, g.s2, level);
 }
 
 // ---- KineticClass::SingleAction link term (KineticClass.cc:45-78) ----

@@ -65,6 +65,7 @@ struct DDavid {
   const R *duy, *dud2;  // dukj [tau][point][col]
   const R *diag;        // column 1 of ukj as (y, d2y) pairs [tau][diag_stride][2]
   int diag_stride;      // points per level of diag, rounded up to an even count
+  const R *est;         // FP64: (V, V'', dU_00, dU_00'') per point, [tau][point][4], for the energy estimator
 };
 
 // PAtricubicFitClass tables for one species pair, one precision.
@@ -182,6 +183,7 @@ struct pimc_context {
   unsigned int *d_counter = nullptr;
   double *d_out = nullptr;
   double *h_out = nullptr;  // pinned
+  float4 *d_bounds = nullptr;  // bounding spheres of the pair sums (pair_path.cu)
   int *d_active = nullptr;
   // bisection
   pimc_bisection_desc bis{};
