@@ -5,6 +5,8 @@
 // over the per-block partials), so results are bitwise reproducible.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "action_kernels.cuh"
 #include "device_math.cuh"
 
@@ -96,15 +98,6 @@ __global__ void __launch_bounds__(256) sr_single_kernel(const double *__restrict
   finish_sum(r, partials, counter, out, sh);
 }
 
-// Triangular pair index k -> (p1, p2) with p2 < p1.
-__device__ __forceinline__ void tri_decode(long long k, int &p1, int &p2) {
-  long long a = (long long)((1.0 + sqrt(1.0 + 8.0 * (double)k)) * 0.5);
-  while (a * (a - 1) / 2 > k) a--;
-  while ((a + 1) * a / 2 <= k) a++;
-  p1 = (int)a;
-  p2 = (int)(k - a * (a - 1) / 2);
-}
-
 // ---- observables: PairCorrelationClass::Accumulate ----
 // PathClass::DistDisp one-slice form (PathClass.h:637-660): minimum image by
 // nearbyint(disp / L), then |disp|.
@@ -120,35 +113,94 @@ __device__ __forceinline__ double dist_one_slice(const double a[3], const double
   return sqrt(d2);
 }
 
-// The g(r) histogram: one pass over slices [0, S-2] x pairs p2 < p1 of the OLD
-// path, pair distances below the grid end in bin
-// (int)nearbyint((r - start) * deltainv - 0.5) (ObservableCorrelation.cc:
-// 191-207, Grid.h:81-84); bins counted per block in shared memory, then added
-// to the 64-bit histogram.
-__global__ void __launch_bounds__(256) gofr_kernel(const double *__restrict__ path, DevSystem sys, GofrGrid gg,
+// The g(r) histogram: slices [0, S-2] x pairs p2 < p1 of the OLD path, pair
+// distances below the grid end in bin (int)nearbyint((r - start) * deltainv -
+// 0.5) (ObservableCorrelation.cc:191-207, Grid.h:81-84); bins counted per block
+// in shared memory, then added to the 64-bit histogram.
+// A block takes (tile of particles) x (tile) x slice items: the tiles'
+// positions are boxed in FP64 and staged as FP32, and a pair's distance and
+// place on the grid are formed in FP32.  The place carries an error below
+// `err` bins (see launch_gofr); a pair nearer than that to a bin's edge, or
+// with a position FP32 cannot box, is binned from its FP64 distance, so the
+// counts are the FP64 evaluation's.  With FP64 distances and 64-bit index
+// arithmetic for every pair this took 138 us for N = 512, M = 128 and 100 bins
+// and was bound by the FP64 and integer work; it now takes 44 us (ncu), bound by
+// instruction issue (about 50 a pair).
+template <int JPL>  // j particles per lane: tiles of 32 JPL particles
+__global__ void __launch_bounds__(256, 4) gofr_kernel(const double *__restrict__ path, DevSystem sys, GofrGrid gg,
+                                                   long long items, float err, float past,
                                                    unsigned long long *hist) {
+  constexpr int T = 32 * JPL;
   extern __shared__ unsigned int s_hist[];
-  const int N = sys.N, S = sys.S;
-  const long long npairs = (long long)N * (N - 1) / 2;
-  const long long total = npairs * (S - 1);
-  for (int i = threadIdx.x; i < gg.nbins; i += blockDim.x) s_hist[i] = 0u;
-  __syncthreads();
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int slice = (int)(idx / npairs);
-    int p1, p2;
-    tri_decode(idx - (long long)slice * npairs, p1, p2);
-    double a[3], b[3];
-    load3(path + ((size_t)slice * N + p1) * 3, a);
-    load3(path + ((size_t)slice * N + p2) * 3, b);
-    const double dist = dist_one_slice(a, b, sys);
-    if (dist < gg.end) {
-      const int bin = (int)rint(rsub(rmul(rsub(dist, gg.start), gg.deltainv), 0.5));
-      if (bin >= 0 && bin < gg.nbins) atomicAdd(&s_hist[bin], 1u);
+  __shared__ float4 s_pos[2 * T];  // the i tile, then the j tile
+  const int N = sys.N, S1 = sys.S - 1, tid = threadIdx.x, lane = tid & 31;
+  for (int i = tid; i < gg.nbins; i += blockDim.x) s_hist[i] = 0u;
+  const float Lx = (float)sys.box[0], Ly = (float)sys.box[1], Lz = (float)sys.box[2];
+  const float ix = (float)sys.boxinv[0], iy = (float)sys.boxinv[1], iz = (float)sys.boxinv[2];
+  const float dinv = (float)gg.deltainv, t0 = (float)(gg.start * gg.deltainv);
+  // A block takes consecutive items, slice fastest, so it divides once.
+  const long long beg = items * blockIdx.x / gridDim.x, end = items * (blockIdx.x + 1) / gridDim.x;
+  int ti, tj, slice = (int)(beg % S1);
+  tri_decode(beg / S1, ti, tj);
+  for (long long item = beg; item < end; item++) {
+    const int i0 = ti * T, j0 = tj * T;
+    const int ni = min(T, N - i0), nj = min(T, N - j0);
+    const double *row = path + (size_t)slice * N * 3;
+    __syncthreads();  // the previous item's readers are done
+    if (tid < 2 * T) {
+      const int p = tid < T ? i0 + tid : j0 + tid - T;
+      if (p < N) {
+        float v[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          const double x = row[(size_t)p * 3 + d], b = sys.box[d];
+          const double boxed = x - round_even_magic(x * sys.boxinv[d]) * b;
+          v[d] = fabs(x) <= 1e6 * b ? (float)boxed : __int_as_float(0x7fffffff);  // NaN: FP64 for its pairs
+        }
+        s_pos[tid] = make_float4(v[0], v[1], v[2], 0.0f);
+      }
+    }
+    __syncthreads();
+    float4 q[JPL];
+#pragma unroll
+    for (int h = 0; h < JPL; h++) q[h] = s_pos[T + lane + 32 * h];
+#pragma unroll 2
+    for (int i = tid >> 5; i < ni; i += 8) {
+      const float4 p = s_pos[i];
+      const int jend = ti == tj ? i : nj;
+#pragma unroll
+      for (int h = 0; h < JPL; h++) {
+        const int j = lane + 32 * h;
+        float dx = q[h].x - p.x, dy = q[h].y - p.y, dz = q[h].z - p.z;
+        dx -= round_even_magic(dx * ix) * Lx;
+        dy -= round_even_magic(dy * iy) * Ly;
+        dz -= round_even_magic(dz * iz) * Lz;
+        float dist;
+        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(dist) : "f"(dx * dx + dy * dy + dz * dz));
+        const float t = dist * dinv - t0;
+        if (t > past || j >= jend) continue;
+        const float low = round_even_magic(t - 0.5f), e = t - low;
+        int bin = int_of_integral(low);
+        if (!(e > err && e < 1.0f - err)) {
+          double a[3], b[3];
+          load3(row + (size_t)(i0 + i) * 3, a);
+          load3(row + (size_t)(j0 + j) * 3, b);
+          const double d64 = dist_one_slice(a, b, sys);
+          bin = d64 < gg.end ? (int)rint(rsub(rmul(rsub(d64, gg.start), gg.deltainv), 0.5)) : -1;
+        }
+        if ((unsigned)bin < (unsigned)gg.nbins) atomicAdd(&s_hist[bin], 1u);
+      }
+    }
+    if (++slice == S1) {
+      slice = 0;
+      if (++tj > ti) {
+        ti++;
+        tj = 0;
+      }
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < gg.nbins; i += blockDim.x)
+  for (int i = tid; i < gg.nbins; i += blockDim.x)
     if (s_hist[i]) atomicAdd(&hist[i], (unsigned long long)s_hist[i]);
 }
 
@@ -304,11 +356,33 @@ cudaError_t launch_kin_dbeta(const ReduceTarget &t, const double *path, const De
   return cudaGetLastError();
 }
 
+// err, in bins, with u = 2^-24: a boxed coordinate rounds by L u / 2; the
+// difference of two by L u, its image by L u (the FP32 box side) + L u / 2: with
+// both coordinates 3.5 L u a dimension, sqrt(3) times that for the distance, and
+// the squares, their sum and the root (2^-22 of itself at most) add 6.5 u of a
+// distance up to 0.87 L; start deltainv rounds by u of itself and the place by 3 u
+// of itself, at most the bins to the box diagonal.  16 L u deltainv + 4 u (nbins + start deltainv)
+// holds them all.  The bound on |x| leaves the FP64 distance's own rounding
+// (1e6 L 2^-52) far below that.  From 1/2 on every pair takes the FP64 path, as
+// for boxes whose squares FP32 does not hold.
 cudaError_t launch_gofr(cudaStream_t st, const double *path, const DevSystem &sys, const GofrGrid &gg,
                         unsigned long long *hist, int sm_count) {
-  const long long items = (long long)sys.N * (sys.N - 1) / 2 * (sys.S - 1);
-  const int blocks = grid_for(items, 256, sm_count);
-  gofr_kernel<<<blocks, 256, (size_t)gg.nbins * sizeof(unsigned int), st>>>(path, sys, gg, hist);
+  const double L = fmax(sys.box[0], fmax(sys.box[1], sys.box[2]));
+  double err = (16.0 * L * gg.deltainv + 4.0 * (gg.nbins + gg.start * gg.deltainv)) * 5.9604644775390625e-8;
+  if (!(L < 1e15 && L > 1e-15)) err = HUGE_VAL;
+  auto count = [&](int tile) {
+    const long long nt = (sys.N + tile - 1) / tile;
+    return nt * (nt + 1) / 2 * (sys.S - 1);
+  };
+  const bool wide = count(64) >= 4 * sm_count;  // tiles of 64 unless they leave the SMs short of blocks
+  const long long items = count(wide ? 64 : 32);
+  const int blocks = (int)std::min(items, (long long)4 * sm_count);  // all resident
+  const size_t dyn = (size_t)gg.nbins * sizeof(unsigned int);
+  auto kfn = wide ? gofr_kernel<2> : gofr_kernel<1>;
+  const cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             12288 * (int)sizeof(unsigned int));  // beside the static tiles
+  if (e != cudaSuccess) return e;
+  kfn<<<blocks, 256, dyn, st>>>(path, sys, gg, items, (float)err, (float)(gg.nbins + 1 + err), hist);
   return cudaGetLastError();
 }
 

@@ -777,6 +777,15 @@ __device__ __forceinline__ MixedU pa_U_mixed(const DevPA &pa, const float2 *diag
   return coulomb_U_mixed(pa.c64, pa.c32, g, level);
 }
 
+// Triangular index k -> (a, b) with b <= a.
+__device__ __forceinline__ void tri_decode(long long k, int &a, int &b) {
+  long long r = (long long)((sqrt(8.0 * (double)k + 1.0) - 1.0) * 0.5);
+  while (r * (r + 1) / 2 > k) r--;
+  while ((r + 1) * (r + 2) / 2 <= k) r++;
+  a = (int)r;
+  b = (int)(k - r * (r + 1) / 2);
+}
+
 // Two-sum accumulation (Knuth): s + c carries the running sum of the terms
 // with the exact rounding error of each FP64 addition gathered in c (FP32
 // suffices for c: each error is below 2^-53 |s|).

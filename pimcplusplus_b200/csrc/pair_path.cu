@@ -106,15 +106,6 @@ __device__ __forceinline__ SliceVal slice_value(const DevPA &pa, const Tables<KI
   return s;
 }
 
-// Triangular index k -> (a, b) with b <= a.
-__device__ __forceinline__ void tri_decode(long long k, int &a, int &b) {
-  long long r = (long long)((sqrt(8.0 * (double)k + 1.0) - 1.0) * 0.5);
-  while (r * (r + 1) / 2 > k) r--;
-  while ((r + 1) * (r + 2) / 2 <= k) r++;
-  a = (int)r;
-  b = (int)(k - r * (r + 1) / 2);
-}
-
 // Displacement b - a in the minimum image (PathClass::DistDisp): raw and boxed.
 __device__ __forceinline__ void displacement(const double *a, const double *b, const DevSystem &s, double raw[3],
                                              double d[3]) {
