@@ -12,7 +12,12 @@
 
 namespace pimc {
 
-// Block-wide sum; the result is valid in thread 0.  `sh` holds >= 32 doubles.
+// Threads per block of the reductions.  Most calls are one window of one
+// particle: a few hundred to a few thousand terms, each a serial chain of FP64
+// operations and dependent loads, so small blocks spread the terms over SMs.
+constexpr int kReduceThreads = 128;
+
+// Block-wide sum; the result is valid in thread 0.  `sh` holds a double per warp.
 __device__ __forceinline__ double block_sum(double v, double *sh) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -21,18 +26,21 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
   if (l == 0) sh[w] = v;
   __syncthreads();
   double r = 0.0;
-  if (threadIdx.x == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    for (int i = 0; i < nw; i++) r += sh[i];
-  }
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int i = 0; i < kReduceThreads / 32; i++) r += sh[i];
   return r;
 }
 
 // Writes this block's partial and lets the last block to finish add all
-// partials in block order into *out.
+// partials in block order into *out.  A single block writes its sum itself.
 __device__ __forceinline__ void finish_sum(double partial, double *partials, unsigned int *counter, double *out,
                                            double *sh) {
   __shared__ int s_last;
+  if (gridDim.x == 1) {
+    if (threadIdx.x == 0) *out = partial;
+    return;
+  }
   if (threadIdx.x == 0) {
     partials[blockIdx.x] = partial;
     __threadfence();
@@ -60,10 +68,10 @@ __device__ __forceinline__ void load3(const double *__restrict__ p, double v[3])
 // ShortRangeClass::SingleAction (ShortRangeClass.cc:191-236).  Item order:
 // active particle, link, partner (partner fastest, for coalesced path reads).
 template <int KIND, typename R>
-__global__ void __launch_bounds__(256) sr_single_kernel(const double *__restrict__ path, DevSystem sys, DevPA pa,
+__global__ void __launch_bounds__(kReduceThreads) sr_single_kernel(const double *__restrict__ path, DevSystem sys, DevPA pa,
                                                         ActiveList act, int slice1, int skip, int nlinks, int level,
                                                         double *partials, unsigned int *counter, double *out) {
-  __shared__ double sh[32];
+  __shared__ double sh[kReduceThreads / 32];
   typedef typename Pair2<R>::T P2;
   const P2 *diag = nullptr;
   if (KIND == PA_DAVID) {
@@ -74,12 +82,22 @@ __global__ void __launch_bounds__(256) sr_single_kernel(const double *__restrict
   const long long per_active = (long long)N * nlinks;
   const long long total = per_active * act.n;
   double acc = 0.0;
+  const bool small = total <= 0x7fffffffll;  // 32-bit divisions: the 64-bit ones are a call each
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
-    const int pi = (int)(idx / per_active);
-    const long long rem = idx - pi * per_active;
-    const int link = (int)(rem / N);
-    const int p2 = (int)(rem - (long long)link * N);
+    int pi, link, p2;
+    if (small) {
+      const unsigned i = (unsigned)idx, pa1 = (unsigned)per_active;
+      pi = act.n == 1 ? 0 : (int)(i / pa1);
+      const unsigned rem = i - (unsigned)pi * pa1;
+      link = (int)(rem / (unsigned)N);
+      p2 = (int)(rem - (unsigned)link * (unsigned)N);
+    } else {
+      pi = (int)(idx / per_active);
+      const long long rem = idx - pi * per_active;
+      link = (int)(rem / N);
+      p2 = (int)(rem - (long long)link * N);
+    }
     const int p1 = act.p[pi];
     bool visited = false;  // Path.DoPtcl: moved particles count once
     for (int k = 0; k <= pi; k++) visited |= (act.p[k] == p2);
@@ -214,10 +232,10 @@ __device__ __forceinline__ void velocity(const double *__restrict__ path, int N,
 }
 
 // KineticClass::SingleAction (KineticClass.cc:33-90)
-__global__ void __launch_bounds__(256) kin_single_kernel(const double *__restrict__ path, DevSystem sys,
+__global__ void __launch_bounds__(kReduceThreads) kin_single_kernel(const double *__restrict__ path, DevSystem sys,
                                                          ActiveList act, int slice1, int skip, int nlinks, int level,
                                                          double *partials, unsigned int *counter, double *out) {
-  __shared__ double sh[32];
+  __shared__ double sh[kReduceThreads / 32];
   const double levelTau = sys.tau * (1 << level);
   const double F = 1.0 / (4.0 * sys.lambda * levelTau);
   const int total = act.n * nlinks;
@@ -235,10 +253,10 @@ __global__ void __launch_bounds__(256) kin_single_kernel(const double *__restric
 }
 
 // KineticClass::d_dBeta (KineticClass.cc:187-256)
-__global__ void __launch_bounds__(256) kin_dbeta_kernel(const double *__restrict__ path, DevSystem sys, int slice1,
+__global__ void __launch_bounds__(kReduceThreads) kin_dbeta_kernel(const double *__restrict__ path, DevSystem sys, int slice1,
                                                         int skip, int nlinks, int level, double *partials,
                                                         unsigned int *counter, double *out) {
-  __shared__ double sh[32];
+  __shared__ double sh[kReduceThreads / 32];
   const double levelTau = ldexp(sys.tau, level);
   const double F = 1.0 / (4.0 * sys.lambda * levelTau);
   const int total = sys.N * nlinks;
@@ -301,40 +319,37 @@ __global__ void reject_kernel(const double *path_old, double *path_new, DevSyste
 // ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------
-static int grid_for(long long items, int threads, int sm_count) {
-  long long b = (items + threads - 1) / threads;
-  long long cap = (long long)sm_count * 8;
-  if (b > cap) b = cap;
-  if (b > kPartialSlots) b = kPartialSlots;
-  if (b < 1) b = 1;
-  return (int)b;
+static int grid_for(long long items, int sm_count) {
+  long long b = (items + kReduceThreads - 1) / kReduceThreads;
+  b = std::min(b, std::min((long long)sm_count * 16, (long long)kPartialSlots));
+  return (int)std::max(b, 1ll);
 }
 
 cudaError_t launch_sr_single(const ReduceTarget &t, const double *path, const DevSystem &sys, const DevPA &pa,
                              const ActiveList &act, int slice1, int skip, int nlinks, int level, int precision,
                              int sm_count) {
   long long items = (long long)act.n * sys.N * nlinks;
-  int blocks = grid_for(items, 256, sm_count);
+  int blocks = grid_for(items, sm_count);
   if (pa.kind == PA_DAVID) {
     if (precision == PIMC_MIXED)
-      sr_single_kernel<PA_DAVID, float><<<blocks, 256, 0, t.stream>>>(path, sys, pa, act, slice1, skip, nlinks, level,
+      sr_single_kernel<PA_DAVID, float><<<blocks, kReduceThreads, 0, t.stream>>>(path, sys, pa, act, slice1, skip, nlinks, level,
                                                                        t.partials, t.counter, t.out);
     else
-      sr_single_kernel<PA_DAVID, double><<<blocks, 256, 0, t.stream>>>(path, sys, pa, act, slice1, skip, nlinks, level,
+      sr_single_kernel<PA_DAVID, double><<<blocks, kReduceThreads, 0, t.stream>>>(path, sys, pa, act, slice1, skip, nlinks, level,
                                                                         t.partials, t.counter, t.out);
   } else if (pa.kind == PA_COULOMB) {
     if (precision == PIMC_MIXED)
-      sr_single_kernel<PA_COULOMB, float><<<blocks, 256, 0, t.stream>>>(path, sys, pa, act, slice1, skip, nlinks,
+      sr_single_kernel<PA_COULOMB, float><<<blocks, kReduceThreads, 0, t.stream>>>(path, sys, pa, act, slice1, skip, nlinks,
                                                                          level, t.partials, t.counter, t.out);
     else
-      sr_single_kernel<PA_COULOMB, double><<<blocks, 256, 0, t.stream>>>(path, sys, pa, act, slice1, skip, nlinks,
+      sr_single_kernel<PA_COULOMB, double><<<blocks, kReduceThreads, 0, t.stream>>>(path, sys, pa, act, slice1, skip, nlinks,
                                                                           level, t.partials, t.counter, t.out);
   } else {
     if (precision == PIMC_MIXED)
-      sr_single_kernel<PA_TRICUBIC, float><<<blocks, 256, 0, t.stream>>>(path, sys, pa, act, slice1, skip, nlinks,
+      sr_single_kernel<PA_TRICUBIC, float><<<blocks, kReduceThreads, 0, t.stream>>>(path, sys, pa, act, slice1, skip, nlinks,
                                                                           level, t.partials, t.counter, t.out);
     else
-      sr_single_kernel<PA_TRICUBIC, double><<<blocks, 256, 0, t.stream>>>(path, sys, pa, act, slice1, skip, nlinks,
+      sr_single_kernel<PA_TRICUBIC, double><<<blocks, kReduceThreads, 0, t.stream>>>(path, sys, pa, act, slice1, skip, nlinks,
                                                                            level, t.partials, t.counter, t.out);
   }
   return cudaGetLastError();
@@ -342,16 +357,16 @@ cudaError_t launch_sr_single(const ReduceTarget &t, const double *path, const De
 
 cudaError_t launch_kin_single(const ReduceTarget &t, const double *path, const DevSystem &sys, const ActiveList &act,
                               int slice1, int skip, int nlinks, int level, int sm_count) {
-  int blocks = grid_for((long long)act.n * nlinks, 256, sm_count);
-  kin_single_kernel<<<blocks, 256, 0, t.stream>>>(path, sys, act, slice1, skip, nlinks, level, t.partials, t.counter,
+  int blocks = grid_for((long long)act.n * nlinks, sm_count);
+  kin_single_kernel<<<blocks, kReduceThreads, 0, t.stream>>>(path, sys, act, slice1, skip, nlinks, level, t.partials, t.counter,
                                                   t.out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_kin_dbeta(const ReduceTarget &t, const double *path, const DevSystem &sys, int slice1, int skip,
                              int nlinks, int level, int sm_count) {
-  int blocks = grid_for((long long)sys.N * nlinks, 256, sm_count);
-  kin_dbeta_kernel<<<blocks, 256, 0, t.stream>>>(path, sys, slice1, skip, nlinks, level, t.partials, t.counter,
+  int blocks = grid_for((long long)sys.N * nlinks, sm_count);
+  kin_dbeta_kernel<<<blocks, kReduceThreads, 0, t.stream>>>(path, sys, slice1, skip, nlinks, level, t.partials, t.counter,
                                                  t.out);
   return cudaGetLastError();
 }

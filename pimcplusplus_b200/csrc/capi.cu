@@ -133,8 +133,10 @@ int check_active(pimc_context *ctx, const int *active, int n, ActiveList &out) {
   return PIMC_OK;
 }
 
+// The reduction kernels write their scalar into pinned host memory themselves
+// (a copy operation behind the kernel costs a few us of a call that takes
+// twenty); it is there once the stream has run dry.
 int finish_scalar(pimc_context *ctx, double *out) {
-  CK(cudaMemcpyAsync(ctx->h_out, ctx->d_out, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   *out = *ctx->h_out;
   if (!std::isfinite(*out)) return fail(ctx, PIMC_E_NAN, "non-finite action");
@@ -248,7 +250,6 @@ int pimc_create(const pimc_system_desc *d, pimc_context **out) {
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_partials, kPartialSlots * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_counter, sizeof(unsigned int));
   if (e == cudaSuccess) e = cudaMemset(ctx->d_counter, 0, sizeof(unsigned int));
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_out, 4 * sizeof(double));
   if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_out, 4 * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_bounds, pair_path_bounds_bytes(s.N, s.S));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_chain, kMaxChainStates * sizeof(ChainState));
@@ -272,7 +273,6 @@ int pimc_destroy(pimc_context *ctx) {
   for (int c = 0; c < 2; c++) cudaFree(ctx->d_path[c]);
   cudaFree(ctx->d_partials);
   cudaFree(ctx->d_counter);
-  cudaFree(ctx->d_out);
   cudaFree(ctx->d_bounds);
   if (ctx->h_out) cudaFreeHost(ctx->h_out);
   cudaFree(ctx->d_chain);
@@ -524,7 +524,7 @@ int pimc_single_action(pimc_context *ctx, int action, int copy, int slice1, int 
   if (action == PIMC_ACTION_DAVIDLONGRANGE) return yk_single(ctx, copy, slice1, slice2, act, level, out);
   const int skip = 1 << level;
   const int nlinks = (slice2 - slice1 + skip - 1) / skip;
-  ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->d_out};
+  ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->h_out};
   const double *path = ctx->d_path[copy];
   if (nlinks == 0 || n_active == 0) {
     *out = 0.0;
@@ -557,17 +557,21 @@ static int longrange_single(pimc_context *ctx, int copy, int slice1, int slice2,
   const int skip = 1 << level;
   if (slice2 > ctx->sys.S - 1) return fail(ctx, PIMC_E_ARG, "slice range out of range");
   const LRDesc lr = lr_desc(ctx);
-  if (copy == PIMC_NEW)
-    CK(launch_rhok_update(ctx->stream, ctx->d_path[0], ctx->d_path[1], ctx->sys.N, lr, act, slice1, slice2, skip,
-                          ctx->d_rhok[0], ctx->d_rhok[1]));
   double ksum = 0.0;
   if (pa_long_range(ctx)) {
-    ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->d_out};
-    CK(launch_lr_sum(t, ctx->d_rhok[copy], lr, ctx->d_ulong_k + (size_t)level * ctx->num_k, slice1, slice2, skip,
-                     ctx->sm_count));
+    ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->h_out};
+    const double *uk = ctx->d_ulong_k + (size_t)level * ctx->num_k;
+    if (copy == PIMC_NEW)
+      CK(launch_rhok_update_sum(t, ctx->d_path[0], ctx->d_path[1], ctx->sys.N, lr, act, slice1, slice2, skip,
+                                ctx->d_rhok[0], ctx->d_rhok[1], uk, ctx->sm_count));
+    else
+      CK(launch_lr_sum(t, ctx->d_rhok[0], lr, uk, slice1, slice2, skip, ctx->sm_count));
     int rc = finish_scalar(ctx, &ksum);
     if (rc) return rc;
   } else {
+    if (copy == PIMC_NEW)
+      CK(launch_rhok_update(ctx->stream, ctx->d_path[0], ctx->d_path[1], ctx->sys.N, lr, act, slice1, slice2, skip,
+                            ctx->d_rhok[0], ctx->d_rhok[1]));
     CK(cudaStreamSynchronize(ctx->stream));
   }
   *out = ksum + lr_constant(ctx, slice1, slice2, level, false);
@@ -590,7 +594,7 @@ int pimc_d_dbeta(pimc_context *ctx, int action, int slice1, int slice2, int leve
     CK(launch_rhok_full(ctx->stream, ctx->d_path[0], ctx->sys.N, ctx->sys.S, lr, ctx->sm_count, ctx->d_rhok[0]));
     double ksum = 0.0;
     if (pa_long_range(ctx)) {
-      ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->d_out};
+      ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->h_out};
       CK(launch_lr_sum(t, ctx->d_rhok[0], lr, ctx->d_dulong_k + (size_t)level * ctx->num_k, slice1, slice2, skip,
                        ctx->sm_count));
       int rc2 = finish_scalar(ctx, &ksum);
@@ -607,7 +611,7 @@ int pimc_d_dbeta(pimc_context *ctx, int action, int slice1, int slice2, int leve
     return PIMC_OK;
   }
   if ((slice1 + (nlinks - 1) * skip + skip) >= ctx->sys.S) return fail(ctx, PIMC_E_ARG, "link runs past the last slice");
-  ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->d_out};
+  ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->h_out};
   const double *path = ctx->d_path[PIMC_OLD];
   switch (action) {
     case PIMC_ACTION_SHORTRANGE:
@@ -1066,16 +1070,20 @@ static int yk_single(pimc_context *ctx, int copy, int slice1, int slice2, const 
   const bool inclusive = !(slice1 == 0 && slice2 == ctx->sys.S - 1);
   const int first = inclusive ? slice1 + skip : slice1, last = slice2 - skip;
   const LRDesc lr = lr_desc(ctx);
-  if (copy == PIMC_NEW && first <= last)
-    CK(launch_rhok_update(ctx->stream, ctx->d_path[0], ctx->d_path[1], ctx->sys.N, lr, act, first, last, skip,
-                          ctx->d_rhok[0], ctx->d_rhok[1]));
   if (act.n == 0 || first > last) {
+    if (copy == PIMC_NEW && first <= last)
+      CK(launch_rhok_update(ctx->stream, ctx->d_path[0], ctx->d_path[1], ctx->sys.N, lr, act, first, last, skip,
+                            ctx->d_rhok[0], ctx->d_rhok[1]));
     CK(cudaStreamSynchronize(ctx->stream));
     *out = 0.0;
     return PIMC_OK;
   }
-  ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->d_out};
-  CK(launch_lr_sum(t, ctx->d_rhok[copy], lr, ctx->d_yk, first, last, skip, ctx->sm_count, 1.0));
+  ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->h_out};
+  if (copy == PIMC_NEW)
+    CK(launch_rhok_update_sum(t, ctx->d_path[0], ctx->d_path[1], ctx->sys.N, lr, act, first, last, skip,
+                              ctx->d_rhok[0], ctx->d_rhok[1], ctx->d_yk, ctx->sm_count, 1.0));
+  else
+    CK(launch_lr_sum(t, ctx->d_rhok[0], lr, ctx->d_yk, first, last, skip, ctx->sm_count, 1.0));
   return finish_scalar(ctx, out);
 }
 
@@ -1086,7 +1094,7 @@ static int yk_sum(pimc_context *ctx, int slice1, int slice2, int table, double *
   if (!ctx->yk_ready) return fail(ctx, PIMC_E_STATE, "pimc_davidlongrange_yk not called");
   const LRDesc lr = lr_desc(ctx);
   CK(launch_rhok_full(ctx->stream, ctx->d_path[0], ctx->sys.N, ctx->sys.S, lr, ctx->sm_count, ctx->d_rhok[0]));
-  ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->d_out};
+  ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->h_out};
   CK(launch_lr_sum(t, ctx->d_rhok[0], lr, ctx->d_yk + (size_t)table * ctx->num_k, slice1, slice2, 1, ctx->sm_count,
                    0.5));
   return finish_scalar(ctx, out);
@@ -1146,21 +1154,20 @@ int pimc_energy(pimc_context *ctx, pimc_energy_terms *out) {
   // another, each into its own scalar, and read back together.
   if (int rc = pa_levels_ok(ctx, 1)) return rc;
   const double *path = ctx->d_path[PIMC_OLD];
-  ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->d_out};
+  ReduceTarget t{ctx->stream, ctx->d_partials, ctx->d_counter, ctx->h_out};
   CK(launch_kin_dbeta(t, path, ctx->sys, 0, 1, M, 0, ctx->sm_count));
-  t.out = ctx->d_out + 1;
+  t.out = ctx->h_out + 1;
   CK(launch_pair_path(t, path, ctx->sys, ctx->pa, 0, 1, M, 0, true, ctx->d_bounds, ctx->sm_count));
   int n = 3;
   if (ctx->lr_ready) {  // LongRangeClass::d_dBeta: rho_k of the OLD copy recomputed
     const LRDesc lr = lr_desc(ctx);
     CK(launch_rhok_full(ctx->stream, path, ctx->sys.N, ctx->sys.S, lr, ctx->sm_count, ctx->d_rhok[0]));
     if (pa_long_range(ctx)) {
-      t.out = ctx->d_out + 3;
+      t.out = ctx->h_out + 3;
       CK(launch_lr_sum(t, ctx->d_rhok[0], lr, ctx->d_dulong_k, 0, M, 1, ctx->sm_count));
       n = 4;
     }
   }
-  CK(cudaMemcpyAsync(ctx->h_out, ctx->d_out, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   for (int i = 0; i < n; i++)
     if (!std::isfinite(ctx->h_out[i])) return fail(ctx, PIMC_E_NAN, "non-finite action");

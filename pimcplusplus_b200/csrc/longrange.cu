@@ -136,48 +136,6 @@ __global__ void __launch_bounds__(256) rhok_full_kernel(const double *__restrict
   cluster.sync();  // no block leaves while a peer reads its sums
 }
 
-// One block per updated slice (slice1 + b*skip): NEW = OLD, then per active
-// particle NEW += C(r_new), NEW -= C(r_old), in the reference's order.
-__global__ void __launch_bounds__(256) rhok_update_kernel(const double *__restrict__ path_old,
-                                                          const double *__restrict__ path_new, int N, LRDesc lr,
-                                                          ActiveList act, int slice1, int skip,
-                                                          const double2 *__restrict__ rho_old, double2 *rho_new) {
-  __shared__ double2 Cn[kMaxPhase], Co[kMaxPhase];
-  const int slice = slice1 + blockIdx.x * skip;
-  const int per = (lr.nk + blockDim.x - 1) / blockDim.x;
-  double2 acc[4];
-  for (int j = 0; j < per; j++) {
-    const int k = threadIdx.x + j * blockDim.x;
-    if (k < lr.nk) acc[j] = rho_old[(size_t)slice * lr.nk + k];
-  }
-  for (int pi = 0; pi < act.n; pi++) {
-    __syncthreads();
-    const int p = act.p[pi];
-    if (threadIdx.x < 3) {
-      fill_phase_table(path_new[((size_t)slice * N + p) * 3 + threadIdx.x], threadIdx.x, lr, Cn);
-    } else if (threadIdx.x >= 32 && threadIdx.x < 35) {
-      fill_phase_table(path_old[((size_t)slice * N + p) * 3 + threadIdx.x - 32], threadIdx.x - 32, lr, Co);
-    }
-    __syncthreads();
-    for (int j = 0; j < per; j++) {
-      const int k = threadIdx.x + j * blockDim.x;
-      if (k < lr.nk) {
-        const int3 ki = lr.kidx[k];
-        const double2 tn = k_term(Cn, lr, ki);
-        acc[j].x += tn.x;
-        acc[j].y += tn.y;
-        const double2 to = k_term(Co, lr, ki);
-        acc[j].x -= to.x;
-        acc[j].y -= to.y;
-      }
-    }
-  }
-  for (int j = 0; j < per; j++) {
-    const int k = threadIdx.x + j * blockDim.x;
-    if (k < lr.nk) rho_new[(size_t)slice * lr.nk + k] = acc[j];
-  }
-}
-
 __device__ __forceinline__ double lr_block_sum(double v, double *sh) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -191,26 +149,10 @@ __device__ __forceinline__ double lr_block_sum(double v, double *sh) {
   return r;
 }
 
-// sum over slices [slice1, slice2] step skip of factor * sum_k |rho_k|^2 u_k
-// (the homologous k-space term); factor 1/2 at the two ends.
-__global__ void __launch_bounds__(256) lr_sum_kernel(const double2 *__restrict__ rhok, LRDesc lr,
-                                                     const double *__restrict__ uk, int slice1, int slice2, int skip,
-                                                     double end_weight, double *partials, unsigned int *counter,
-                                                     double *out) {
+// This block's partial, and the last block's sum of all partials in block order.
+__device__ __forceinline__ void lr_finish(double acc, double *partials, unsigned int *counter, double *out) {
   __shared__ double sh[32];
   __shared__ int s_last;
-  const int nsl = (slice2 - slice1) / skip + 1;
-  const long long total = (long long)nsl * lr.nk;
-  double acc = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int b = (int)(i / lr.nk), k = (int)(i - (long long)b * lr.nk);
-    const int slice = slice1 + b * skip;
-    const double factor = (slice == slice1 || slice == slice2) ? end_weight : 1.0;
-    const double2 r = rhok[(size_t)slice * lr.nk + k];
-    const double rhok2 = r.x * r.x + r.y * r.y;
-    acc += factor * 0.5 * 2.0 * rhok2 * uk[k];
-  }
   const double v = lr_block_sum(acc, sh);
   if (threadIdx.x == 0) {
     partials[blockIdx.x] = v;
@@ -227,6 +169,83 @@ __global__ void __launch_bounds__(256) lr_sum_kernel(const double2 *__restrict__
     *out = tot;
     *counter = 0u;
   }
+}
+
+// One block per updated slice (slice1 + b*skip): NEW = OLD, then per active
+// particle NEW += C(r_new), NEW -= C(r_old), in the reference's order.  SUM: the
+// k sum of lr_sum_kernel over the updated slices in the same launch, from the
+// values in registers (LongRangeClass::SingleAction on the NEW copy).
+template <bool SUM>
+__global__ void __launch_bounds__(256) rhok_update_kernel(const double *__restrict__ path_old,
+                                                          const double *__restrict__ path_new, int N, LRDesc lr,
+                                                          ActiveList act, int slice1, int skip,
+                                                          const double2 *__restrict__ rho_old, double2 *rho_new,
+                                                          const double *__restrict__ uk, int slice2,
+                                                          double end_weight, double *partials,
+                                                          unsigned int *counter, double *out) {
+  __shared__ double2 Cn[kMaxPhase], Co[kMaxPhase];
+  const int slice = slice1 + blockIdx.x * skip;
+  double2 acc[4];  // this thread's k-vectors (nk <= 1024)
+  int3 ki[4];
+  double u[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const int k = threadIdx.x + j * blockDim.x;
+    if (k >= lr.nk) break;
+    acc[j] = rho_old[(size_t)slice * lr.nk + k];
+    ki[j] = lr.kidx[k];
+    u[j] = SUM ? uk[k] : 0.0;
+  }
+  for (int pi = 0; pi < act.n; pi++) {
+    __syncthreads();
+    const int p = act.p[pi];
+    if (threadIdx.x < 3) {
+      fill_phase_table(path_new[((size_t)slice * N + p) * 3 + threadIdx.x], threadIdx.x, lr, Cn);
+    } else if (threadIdx.x >= 32 && threadIdx.x < 35) {
+      fill_phase_table(path_old[((size_t)slice * N + p) * 3 + threadIdx.x - 32], threadIdx.x - 32, lr, Co);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if ((int)threadIdx.x + j * (int)blockDim.x >= lr.nk) break;
+      const double2 tn = k_term(Cn, lr, ki[j]);
+      acc[j].x += tn.x;
+      acc[j].y += tn.y;
+      const double2 to = k_term(Co, lr, ki[j]);
+      acc[j].x -= to.x;
+      acc[j].y -= to.y;
+    }
+  }
+  double sum = 0.0;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const int k = threadIdx.x + j * blockDim.x;
+    if (k >= lr.nk) break;
+    rho_new[(size_t)slice * lr.nk + k] = acc[j];
+    if (SUM) sum += (acc[j].x * acc[j].x + acc[j].y * acc[j].y) * u[j];
+  }
+  if (SUM) lr_finish(slice == slice1 || slice == slice2 ? sum * end_weight : sum, partials, counter, out);
+}
+
+// sum over slices [slice1, slice2] step skip of factor * sum_k |rho_k|^2 u_k
+// (the homologous k-space term); factor 1/2 at the two ends.
+__global__ void __launch_bounds__(256) lr_sum_kernel(const double2 *__restrict__ rhok, LRDesc lr,
+                                                     const double *__restrict__ uk, int slice1, int slice2, int skip,
+                                                     double end_weight, double *partials, unsigned int *counter,
+                                                     double *out) {
+  const int nsl = (slice2 - slice1) / skip + 1;
+  const long long total = (long long)nsl * lr.nk;
+  double acc = 0.0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
+       i += (long long)gridDim.x * blockDim.x) {
+    const int b = (int)(i / lr.nk), k = (int)(i - (long long)b * lr.nk);
+    const int slice = slice1 + b * skip;
+    const double factor = (slice == slice1 || slice == slice2) ? end_weight : 1.0;
+    const double2 r = rhok[(size_t)slice * lr.nk + k];
+    const double rhok2 = r.x * r.x + r.y * r.y;
+    acc += factor * 0.5 * 2.0 * rhok2 * uk[k];
+  }
+  lr_finish(acc, partials, counter, out);
 }
 
 __global__ void rhok_copy_kernel(const double2 *__restrict__ src, double2 *dst, int nk, int slice1, int nslices) {
@@ -270,7 +289,23 @@ cudaError_t launch_rhok_update(cudaStream_t st, const double *path_old, const do
                                const LRDesc &lr, const ActiveList &act, int slice1, int slice2, int skip,
                                const double2 *rho_old, double2 *rho_new) {
   const int nsl = (slice2 - slice1) / skip + 1;
-  rhok_update_kernel<<<nsl, 256, 0, st>>>(path_old, path_new, N, lr, act, slice1, skip, rho_old, rho_new);
+  rhok_update_kernel<false><<<nsl, 256, 0, st>>>(path_old, path_new, N, lr, act, slice1, skip, rho_old, rho_new,
+                                                 nullptr, 0, 0.0, nullptr, nullptr, nullptr);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_rhok_update_sum(const ReduceTarget &t, const double *path_old, const double *path_new, int N,
+                                   const LRDesc &lr, const ActiveList &act, int slice1, int slice2, int skip,
+                                   const double2 *rho_old, double2 *rho_new, const double *uk, int sm_count,
+                                   double end_weight) {
+  const int nsl = (slice2 - slice1) / skip + 1;
+  if (nsl > kPartialSlots) {  // a partial a slice
+    const cudaError_t e = launch_rhok_update(t.stream, path_old, path_new, N, lr, act, slice1, slice2, skip, rho_old,
+                                             rho_new);
+    return e != cudaSuccess ? e : launch_lr_sum(t, rho_new, lr, uk, slice1, slice2, skip, sm_count, end_weight);
+  }
+  rhok_update_kernel<true><<<nsl, 256, 0, t.stream>>>(path_old, path_new, N, lr, act, slice1, skip, rho_old, rho_new,
+                                                      uk, slice2, end_weight, t.partials, t.counter, t.out);
   return cudaGetLastError();
 }
 

@@ -181,8 +181,7 @@ struct pimc_context {
   // reduction scratch
   double *d_partials = nullptr;
   unsigned int *d_counter = nullptr;
-  double *d_out = nullptr;
-  double *h_out = nullptr;  // pinned
+  double *h_out = nullptr;  // pinned, written by the reduction kernels
   float4 *d_bounds = nullptr;  // bounding spheres of the pair sums (pair_path.cu)
   int *d_active = nullptr;
   // bisection
