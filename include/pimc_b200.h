@@ -254,7 +254,7 @@ typedef struct pimc_bisection_desc {
   int use_longrange;                /* LongRange pushed at the lowest level */
   int precision;                    /* PIMC_FP64 or PIMC_MIXED */
   int shadow;                       /* also evaluate the other precision, for dS error */
-  int cluster_ctas;                 /* CTAs cooperating on one chain (1..16), 0 = auto;
+  int cluster_ctas;                 /* CTAs cooperating on one chain (1..16), 0 = auto (by N, levels and schedule);
                                        PROPOSALS: proposal slots per window (2..16), one CTA each */
   int threads_per_cta;              /* 0 = auto */
   int schedule;                     /* PIMC_SCHEDULE_SEQUENTIAL, _WINDOWS or _PROPOSALS */

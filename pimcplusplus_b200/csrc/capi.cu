@@ -663,6 +663,45 @@ static int window_slots(const pimc_context *ctx, int num_levels) {
   return std::max(0, std::min(w, kMaxWindows));
 }
 
+// The launch shape of cluster_ctas = 0 / threads_per_cta = 0.  A stage is a
+// latency chain with a fixed part of a few us, so a window is spread until its
+// lowest stage leaves about two terms to a thread: more CTAs only lengthen the
+// exchange of the sums.  `work` counts that stage's pair items, and its k-vector
+// items twice.  Measured per move of the sequential schedule (us; L = 3 unless
+// said), at 1 x 256 / 8 x 256 / 8 x 512 / 16 x 512 CTAs x threads:
+//   1-D table, N = 16 (work 120): 8.5 (4 x 256: 8.5) / 8.6 / 8.9 / 9.9
+//   N = 64 (504): 13.5 / 9.4 / 9.7 / 10.8;  N = 128 (1016): 20.0 / 10.1 / 10.2 / 11.2
+//   N = 64, L = 5 (2016): 15.0 / 10.8 / 8.8 / 9.8;  N = 512 (4088): 48.2 / 13.8 / 11.9 / 11.3
+//   tricubic N = 64: 27.1 / 12.0 / 12.5 / 13.9;  N = 200 (1592): 65 / 17.0 / 13.8 / 14.6;  N = 512: 151 / 28.0 / 20.1 / 17.2
+//   jellium N = 32 (2.4e3): 17.8 / 12.6 / 13.0 / 13.7;  N = 128 (1.0e4): 42.3 / 15.4 / 14.6 / 13.8
+// With concurrent windows the clusters are halved until every window's fits on
+// the GPU at once: a second wave costs more (N = 64, L = 1, 32 windows: 4 x 256
+// 6.2, 8 x 512 17.1).  Proposals keep 8 slots.
+static int auto_launch(pimc_context *ctx) {
+  pimc_bisection_desc &b = ctx->bis;
+  const bool prop = b.schedule == PIMC_SCHEDULE_PROPOSALS;
+  const double work = (double)(ctx->sys.N - 1) * (1 << b.num_levels) +
+                      (b.use_longrange ? 2.0 * ctx->num_k * ((1 << b.num_levels) + 1) : 0.0);
+  if (b.threads_per_cta == 0) b.threads_per_cta = !prop && work > 1200.0 ? 512 : 256;
+  if (b.cluster_ctas != 0) return PIMC_OK;
+  b.cluster_ctas = prop ? 8 : work > 4000.0 ? 16 : work > 200.0 ? 8 : 4;
+  if (prop) return PIMC_OK;
+  const int windows = b.schedule == PIMC_SCHEDULE_SEQUENTIAL ? 1 : window_slots(ctx, b.num_levels);
+  BisectionArgs a{};
+  a.pa = ctx->pa;
+  a.num_levels = b.num_levels;
+  a.proposals = 1;
+  for (; b.cluster_ctas > 1; b.cluster_ctas >>= 1) {
+    int fit = 0;
+    if (bisection_occupancy(a, b.precision, b.shadow, b.cluster_ctas, b.threads_per_cta, &fit) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
+    if (fit >= windows) break;
+  }
+  return PIMC_OK;
+}
+
 int pimc_bisection_setup(pimc_context *ctx, const pimc_bisection_desc *d) {
   if (!ctx || !d) return PIMC_E_ARG;
   if (ctx->pa.kind == PA_NONE) return fail(ctx, PIMC_E_STATE, "no pair action set");
@@ -715,9 +754,7 @@ int pimc_bisection_setup(pimc_context *ctx, const pimc_bisection_desc *d) {
   }
   CK(cudaSetDevice(ctx->device));
   ctx->bis = *d;
-  if (ctx->bis.cluster_ctas == 0)
-    ctx->bis.cluster_ctas = (ctx->sys.N >= 256 || d->schedule == PIMC_SCHEDULE_PROPOSALS) ? 8 : 1;
-  if (ctx->bis.threads_per_cta == 0) ctx->bis.threads_per_cta = 256;
+  if (int rc2 = auto_launch(ctx)) return rc2;
   std::vector<ChainState> cs(kMaxChainStates);
   CK(cudaMemcpy(cs.data(), ctx->d_chain, cs.size() * sizeof(ChainState), cudaMemcpyDeviceToHost));
   for (auto &c : cs) {
