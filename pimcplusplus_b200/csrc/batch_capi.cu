@@ -64,8 +64,8 @@ int bupload(pimc_batch *b, const std::vector<T> &host, const T **dev) {
   void *p = nullptr;
   BCK(cudaMalloc(&p, host.size() * sizeof(T) + 16));
   b->owned.push_back(p);
-  BCK(cudaMemset(p, 0, host.size() * sizeof(T) + 16));
-  BCK(cudaMemcpy(p, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice));
+  BCK(cudaMemsetAsync(p, 0, host.size() * sizeof(T) + 16, b->stream));
+  BCK(cudaMemcpyAsync(p, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice, b->stream));
   *dev = static_cast<const T *>(p);
   return PIMC_OK;
 }
@@ -177,7 +177,7 @@ int pimc_batch_create(int device, int n_chains, const pimc_chain_desc *chains, p
   b->dyn = maxdyn;  // FP64 pairs; see batch_dyn for the other configurations
   e = cudaMalloc(&b->d_paths, total * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_chains, n_chains * sizeof(ChainState));
-  if (e == cudaSuccess) e = cudaMemset(b->d_chains, 0, n_chains * sizeof(ChainState));
+  if (e == cudaSuccess) e = cudaMemsetAsync(b->d_chains, 0, n_chains * sizeof(ChainState), b->stream);
   if (e == cudaSuccess) e = cudaMalloc(&b->d_jobs, n_chains * sizeof(BisectionArgs));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_order, n_chains * sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_queue, sizeof(unsigned int));
@@ -191,8 +191,11 @@ int pimc_batch_create(int device, int n_chains, const pimc_chain_desc *chains, p
   b->jobs.resize(n_chains);
   for (int i = 0; i < n_chains; i++) {
     const pimc_chain_desc &c = chains[i];
-    e = cudaMemcpy(b->d_paths + b->path_off[i], c.path,
-                   (size_t)c.num_time_slices * c.num_particles * 3 * sizeof(double), cudaMemcpyHostToDevice);
+    // set-up copies on the batch's stream (it does not wait for the legacy default
+    // stream), all complete before this call returns
+    e = cudaMemcpyAsync(b->d_paths + b->path_off[i], c.path,
+                        (size_t)c.num_time_slices * c.num_particles * 3 * sizeof(double), cudaMemcpyHostToDevice,
+                        b->stream);
     if (e != cudaSuccess) {
       pimc_batch_destroy(b);
       return PIMC_E_CUDA;
@@ -250,9 +253,10 @@ int pimc_batch_create(int device, int n_chains, const pimc_chain_desc *chains, p
   for (int i = 0; i < n_chains; i++)
     b->cost_sorted[i] =
         (double)chains[order[i]].num_particles * (1 << chains[order[i]].num_levels) * chains[order[i]].steps_per_block;
-  e = cudaMemcpy(b->d_jobs, b->jobs.data(), n_chains * sizeof(BisectionArgs), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_order, order.data(), n_chains * sizeof(int), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_chains, cs.data(), n_chains * sizeof(ChainState), cudaMemcpyHostToDevice);
+  e = cudaMemcpyAsync(b->d_jobs, b->jobs.data(), n_chains * sizeof(BisectionArgs), cudaMemcpyHostToDevice, b->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_order, order.data(), n_chains * sizeof(int), cudaMemcpyHostToDevice, b->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_chains, cs.data(), n_chains * sizeof(ChainState), cudaMemcpyHostToDevice, b->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
   if (e != cudaSuccess) {
     pimc_batch_destroy(b);
     return PIMC_E_CUDA;
@@ -507,7 +511,9 @@ int pimc_batch_set_guard(pimc_batch *b, int guard) {
   BCK(cudaSetDevice(b->device));
   BCK(cudaStreamSynchronize(b->stream));
   for (auto &j : b->jobs) j.guard = guard_mode(guard);
-  BCK(cudaMemcpy(b->d_jobs, b->jobs.data(), b->jobs.size() * sizeof(BisectionArgs), cudaMemcpyHostToDevice));
+  BCK(cudaMemcpyAsync(b->d_jobs, b->jobs.data(), b->jobs.size() * sizeof(BisectionArgs), cudaMemcpyHostToDevice,
+                      b->stream));
+  BCK(cudaStreamSynchronize(b->stream));
   drop_graph(b);
   b->cfg_version++;
   return PIMC_OK;
@@ -517,8 +523,10 @@ int pimc_batch_get_path(pimc_batch *b, int chain, double *path) {
   if (!b || !path || chain < 0 || chain >= b->n_chains) return PIMC_E_ARG;
   BCK(cudaSetDevice(b->device));
   const pimc_chain_desc &c = b->desc[chain];
-  BCK(cudaMemcpy(path, b->d_paths + b->path_off[chain],
-                 (size_t)c.num_time_slices * c.num_particles * 3 * sizeof(double), cudaMemcpyDeviceToHost));
+  BCK(cudaMemcpyAsync(path, b->d_paths + b->path_off[chain],
+                      (size_t)c.num_time_slices * c.num_particles * 3 * sizeof(double), cudaMemcpyDeviceToHost,
+                      b->stream));
+  BCK(cudaStreamSynchronize(b->stream));
   return PIMC_OK;
 }
 

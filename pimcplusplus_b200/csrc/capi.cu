@@ -35,15 +35,24 @@ int cuda_fail(pimc_context *c, cudaError_t e, const char *where) {
     if (e_ != cudaSuccess) return cuda_fail(ctx, e_, #call); \
   } while (0)
 
+// A set-up copy between host and device, complete on return.  On the context's
+// stream: that stream does not wait for the legacy default stream, and a
+// cudaMemcpy from pageable memory returns while its last transfer is under way,
+// so a kernel launched behind it could read what was there before.
+cudaError_t copy_sync(pimc_context *ctx, void *dst, const void *src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, ctx->stream);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(ctx->stream);
+}
+
 template <typename T>
 int upload(pimc_context *ctx, const T *host, size_t n, const T **dev, size_t pad_bytes = 16) {
   void *p = nullptr;
   cudaError_t e = cudaMalloc(&p, n * sizeof(T) + pad_bytes);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(table)");
   ctx->owned.push_back(p);
-  e = cudaMemset(p, 0, n * sizeof(T) + pad_bytes);
+  e = cudaMemsetAsync(p, 0, n * sizeof(T) + pad_bytes, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemset(table)");
-  e = cudaMemcpy(p, host, n * sizeof(T), cudaMemcpyHostToDevice);
+  e = copy_sync(ctx, p, host, n * sizeof(T));
   if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemcpy(table)");
   *dev = static_cast<const T *>(p);
   return PIMC_OK;
@@ -249,14 +258,14 @@ int pimc_create(const pimc_system_desc *d, pimc_context **out) {
   for (int c = 0; c < 2 && e == cudaSuccess; c++) e = cudaMalloc(&ctx->d_path[c], ctx->path_elems * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_partials, kPartialSlots * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_counter, sizeof(unsigned int));
-  if (e == cudaSuccess) e = cudaMemset(ctx->d_counter, 0, sizeof(unsigned int));
+  if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned int), ctx->stream);
   if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_out, 4 * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_bounds, pair_path_bounds_bytes(s.N, s.S));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_chain, kMaxChainStates * sizeof(ChainState));
-  if (e == cudaSuccess) e = cudaMemset(ctx->d_chain, 0, kMaxChainStates * sizeof(ChainState));
+  if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_chain, 0, kMaxChainStates * sizeof(ChainState), ctx->stream);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, d->device);
-  if (e == cudaSuccess) e = cudaMemset(ctx->d_path[0], 0, ctx->path_elems * sizeof(double));
-  if (e == cudaSuccess) e = cudaMemset(ctx->d_path[1], 0, ctx->path_elems * sizeof(double));
+  if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_path[0], 0, ctx->path_elems * sizeof(double), ctx->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_path[1], 0, ctx->path_elems * sizeof(double), ctx->stream);
   if (e != cudaSuccess) {
     pimc_destroy(ctx);
     return PIMC_E_CUDA;
@@ -748,7 +757,7 @@ int pimc_bisection_setup(pimc_context *ctx, const pimc_bisection_desc *d) {
     CK(cudaMalloc(&ctx->d_nbr_cnt, (size_t)ctx->sys.N * sizeof(int)));
     CK(cudaMalloc(&ctx->d_nbr_idx, (size_t)ctx->sys.N * kmax * sizeof(int)));
     CK(cudaMalloc(&ctx->d_nbr_dirty, sizeof(int)));
-    CK(cudaMemset(ctx->d_nbr_dirty, 0xff, sizeof(int)));
+    CK(cudaMemsetAsync(ctx->d_nbr_dirty, 0xff, sizeof(int), ctx->stream));
     ctx->nbr_kmax = kmax;
     ctx->nbr_range = ctx->pa.d64.grid.end;  // the table is zero from its last point on
   }
@@ -756,12 +765,12 @@ int pimc_bisection_setup(pimc_context *ctx, const pimc_bisection_desc *d) {
   ctx->bis = *d;
   if (int rc2 = auto_launch(ctx)) return rc2;
   std::vector<ChainState> cs(kMaxChainStates);
-  CK(cudaMemcpy(cs.data(), ctx->d_chain, cs.size() * sizeof(ChainState), cudaMemcpyDeviceToHost));
+  CK(copy_sync(ctx, cs.data(), ctx->d_chain, cs.size() * sizeof(ChainState)));
   for (auto &c : cs) {
     c.moves = c.accepted = c.stages = c.pair_evals = c.flips = c.redone = c.reevals = 0;
     c.status = 0;
   }
-  CK(cudaMemcpy(ctx->d_chain, cs.data(), cs.size() * sizeof(ChainState), cudaMemcpyHostToDevice));
+  CK(copy_sync(ctx, ctx->d_chain, cs.data(), cs.size() * sizeof(ChainState)));
   ctx->bis_ready = true;
   return PIMC_OK;
 }
@@ -770,7 +779,7 @@ int pimc_rng_seed(pimc_context *ctx, uint64_t seed) {
   if (!ctx) return PIMC_E_ARG;
   CK(cudaSetDevice(ctx->device));
   std::vector<ChainState> cs(kMaxChainStates);
-  CK(cudaMemcpy(cs.data(), ctx->d_chain, cs.size() * sizeof(ChainState), cudaMemcpyDeviceToHost));
+  CK(copy_sync(ctx, cs.data(), ctx->d_chain, cs.size() * sizeof(ChainState)));
   for (int w = 0; w < kMaxChainStates; w++) {
     cs[w].seed = seed;
     cs[w].nlocal = 0;
@@ -784,7 +793,7 @@ int pimc_rng_seed(pimc_context *ctx, uint64_t seed) {
   ctx->rounds = 0;
   ctx->seed = seed;
   ctx->shift_draws = 0;
-  CK(cudaMemcpy(ctx->d_chain, cs.data(), cs.size() * sizeof(ChainState), cudaMemcpyHostToDevice));
+  CK(copy_sync(ctx, ctx->d_chain, cs.data(), cs.size() * sizeof(ChainState)));
   return PIMC_OK;
 }
 
@@ -896,9 +905,9 @@ int pimc_run_bisection(pimc_context *ctx, int n_blocks, pimc_move_record *trace,
     // The status belongs to this call: clear it so that the next call on the
     // context starts clean (the chains' counters and streams are kept).
     std::vector<ChainState> cs(kMaxChainStates);
-    CK(cudaMemcpy(cs.data(), ctx->d_chain, cs.size() * sizeof(ChainState), cudaMemcpyDeviceToHost));
+    CK(copy_sync(ctx, cs.data(), ctx->d_chain, cs.size() * sizeof(ChainState)));
     for (auto &c : cs) c.status = 0;
-    CK(cudaMemcpy(ctx->d_chain, cs.data(), cs.size() * sizeof(ChainState), cudaMemcpyHostToDevice));
+    CK(copy_sync(ctx, ctx->d_chain, cs.data(), cs.size() * sizeof(ChainState)));
     return fail(ctx, st.status, std::string("device status: ") + pimc_status_string(st.status));
   }
   return PIMC_OK;
@@ -981,7 +990,7 @@ int pimc_setup_kvecs(pimc_context *ctx, double kcutoff, int *num_k) {
   cudaFree(ctx->d_kvec);
   ctx->d_kvec = nullptr;
   CK(cudaMalloc(&ctx->d_kvec, ctx->kvecs.size() * sizeof(double) + 16));
-  CK(cudaMemcpy(ctx->d_kvec, ctx->kvecs.data(), ctx->kvecs.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CK(copy_sync(ctx, ctx->d_kvec, ctx->kvecs.data(), ctx->kvecs.size() * sizeof(double)));
   cudaFree(ctx->d_kidx);
   cudaFree(ctx->d_rhok[0]);
   cudaFree(ctx->d_rhok[1]);
@@ -989,10 +998,10 @@ int pimc_setup_kvecs(pimc_context *ctx, double kcutoff, int *num_k) {
   ctx->d_rhok[0] = ctx->d_rhok[1] = nullptr;
   if (ctx->num_k > 0) {
     CK(cudaMalloc(&ctx->d_kidx, kidx.size() * sizeof(int3)));
-    CK(cudaMemcpy(ctx->d_kidx, kidx.data(), kidx.size() * sizeof(int3), cudaMemcpyHostToDevice));
+    CK(copy_sync(ctx, ctx->d_kidx, kidx.data(), kidx.size() * sizeof(int3)));
     for (int c = 0; c < 2; c++) {
       CK(cudaMalloc(&ctx->d_rhok[c], (size_t)ctx->sys.S * ctx->num_k * sizeof(double2)));
-      CK(cudaMemset(ctx->d_rhok[c], 0, (size_t)ctx->sys.S * ctx->num_k * sizeof(double2)));
+      CK(cudaMemsetAsync(ctx->d_rhok[c], 0, (size_t)ctx->sys.S * ctx->num_k * sizeof(double2), ctx->stream));
     }
   }
   *num_k = ctx->num_k;
@@ -1021,8 +1030,8 @@ int pimc_set_longrange(pimc_context *ctx, int num_levels, const double *ulong_k,
   ctx->d_ulong_k = ctx->d_dulong_k = nullptr;
   CK(cudaMalloc(&ctx->d_ulong_k, n * sizeof(double)));
   CK(cudaMalloc(&ctx->d_dulong_k, n * sizeof(double)));
-  CK(cudaMemcpy(ctx->d_ulong_k, ulong_k, n * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ctx->d_dulong_k, dulong_k, n * sizeof(double), cudaMemcpyHostToDevice));
+  CK(copy_sync(ctx, ctx->d_ulong_k, ulong_k, n * sizeof(double)));
+  CK(copy_sync(ctx, ctx->d_dulong_k, dulong_k, n * sizeof(double)));
   ctx->ulong_r0.assign(ulong_r0, ulong_r0 + num_levels);
   ctx->ushort_k0.assign(ushort_k0, ushort_k0 + num_levels);
   ctx->ulong_k0.assign(ulong_k0, ulong_k0 + num_levels);
@@ -1090,7 +1099,7 @@ int pimc_davidlongrange_yk(pimc_context *ctx, int num_kvals, const double *kvals
   ctx->d_yk = nullptr;
   ctx->yk_ready = false;
   CK(cudaMalloc(&ctx->d_yk, t.size() * sizeof(double)));
-  CK(cudaMemcpy(ctx->d_yk, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CK(copy_sync(ctx, ctx->d_yk, t.data(), t.size() * sizeof(double)));
   ctx->yk_ready = true;
   return PIMC_OK;
 }
@@ -1175,7 +1184,7 @@ int pimc_get_rhok(pimc_context *ctx, int copy, double *out) {
   if (!ctx || !out || copy < 0 || copy > 1) return PIMC_E_ARG;
   if (ctx->num_k <= 0) return fail(ctx, PIMC_E_STATE, "pimc_setup_kvecs not called");
   CK(cudaSetDevice(ctx->device));
-  CK(cudaMemcpy(out, ctx->d_rhok[copy], (size_t)ctx->sys.S * ctx->num_k * sizeof(double2), cudaMemcpyDeviceToHost));
+  CK(copy_sync(ctx, out, ctx->d_rhok[copy], (size_t)ctx->sys.S * ctx->num_k * sizeof(double2)));
   return PIMC_OK;
 }
 
