@@ -11,10 +11,21 @@
 //    positions and decisions are identical in every CTA without
 //    communication.  Only the stage action sums cross CTAs: warp 0 stores
 //    this CTA's partials into every peer's shared memory (st.async, each
-//    store completing bytes on the peer's mbarrier); once its mbarrier has
-//    all CTAs' bytes, warp 0 of every CTA adds the partials in rank order —
-//    the same bits everywhere — while the other warps wait at the CTA
-//    barrier only, not at a cluster barrier.
+//    store completing bytes on the peer's mbarrier, one (peer, value) a lane);
+//    once its mbarrier has all CTAs' bytes, warp 0 of every CTA adds the
+//    partials in one order — the same bits everywhere — while the other warps
+//    wait at the CTA barrier only, not at a cluster barrier.
+//  * What bounds it: a stage is one latency chain (terms, sums, exchange,
+//    decision), and a warp on straight-line code that no other warp has just
+//    run issues an instruction every six or seven cycles, so instructions on
+//    the chain count more than arithmetic.  Hence: warp 0 waits for the
+//    evaluating warps' sums and, only before it commits, for the samplers
+//    (two named barriers, so a sampler may take longer than the terms); counters
+//    and records are the sampler warp's; per-level constants are formed once a
+//    job; quotients by an FP32 reciprocal; cells and images by magic-constant
+//    rounding on the FP64 pipe.  A stage of a 64-atom chain on 8 x 256 threads
+//    took 7100 cycles (terms 4000, then 3000 to the next stage) and takes 5900
+//    with the stamps it was measured by (terms 2900).
 //  * Gaussians come from a warp-parallel polar method that reproduces the
 //    sequential draw order exactly (warp_gaussians); the per-midpoint work
 //    of a level runs one midpoint per lane.
@@ -118,6 +129,24 @@ __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// Sums of a and of b over the warp at once: a's in lanes 0-15, b's in 16-31.
+__device__ __forceinline__ double warp_sum_pair(double a, double b, int lane) {
+  const bool hi = lane >= 16;
+  double v = (hi ? b : a) + __shfl_xor_sync(0xffffffffu, hi ? a : b, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// The cluster barrier in halves (all threads of all its CTAs).  Release: the
+// thread's writes are ordered before the barrier; a thread that wrote nothing
+// for the others arrives relaxed and skips that flush.
+__device__ __forceinline__ void cluster_arrive(bool release) {
+  if (release)
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  else
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // warp_sum when only lanes [0, n) can hold nonzero values: the butterfly
 // starts at the half of the smallest power of two >= n (the steps skipped
 // would add exact zeros to lane 0, so lane 0's sum has the same bits), and
@@ -129,22 +158,60 @@ __device__ __forceinline__ double warp_sum_n(double v, int n) {
   return __shfl_sync(0xffffffffu, v, 0);
 }
 
+// 1 / d to an ulp or two, one instruction (the rounded forms are subroutines).
+__device__ __forceinline__ float rcp_approx(float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  return r;
+}
+// floor(n / d) for 0 <= n, 1 <= d < 2^20: below 2^20 by the FP32 reciprocal,
+// whose quotient is off by one at most (n d^-1 carries 4 units of 2^-24); an
+// integer division is a chain several times as long, on the critical path of a stage.
+__device__ __forceinline__ int div_fast(int n, int d) {
+  if (n >= (1 << 20)) return n / d;
+  const int q = (int)((float)n * rcp_approx((float)d));
+  const int r = n - q * d;
+  return r < 0 ? q - 1 : r >= d ? q + 1 : q;
+}
+// floor(it / np) for quotients up to 65 (links or slices of a window), rnp =
+// rcp_approx(np): off by one at most for any it.
+__device__ __forceinline__ int link_of(int it, int np, float rnp) {
+  const int q = (int)((float)it * rnp);
+  const int r = it - q * np;
+  return r < 0 ? q - 1 : r >= np ? q + 1 : q;
+}
+
+// Per level: the sampling width, its square, 1 / (2 sigma^2), and the kinetic
+// action's 1 / (4 lambda tau_l), formed once a job (a division or a root is 80-100
+// cycles of a stage's chain).
+struct LevelConst {
+  double sigma, sigma2, half_inv, kinF;
+};
+__device__ __forceinline__ LevelConst level_const(const DevSystem &s, int level) {
+  LevelConst c;
+  const double levelTau = 0.5 * s.tau * (1 << (level + 1));
+  c.sigma2 = (1.0 * s.lambda * levelTau);
+  c.sigma = sqrt(c.sigma2);
+  c.half_inv = 0.5 / c.sigma2;
+  c.kinF = 1.0 / (4.0 * s.lambda * (s.tau * (1 << level)));
+  return c;
+}
+
 // BisectionStageClass::Sample (BisectionStage.cc:128-289) for one level on
-// the window held in shared memory, run by one full warp: writes the NEW
-// midpoints and returns log T_old - log T_new (identical in every lane).
-__device__ __forceinline__ double sample_level_warp(double (*w_old)[3], double (*w_new)[3], double *gbuf, int num_levels, int level,
-                                    const DevSystem &s, DevRandom &rng, int lane) {
+// the window held in shared memory, run by one full warp, from the unit
+// Gaussians in gbuf: writes the NEW midpoints and returns log T_old - log T_new
+// (identical in every lane).  Out of line: one copy for the three callers keeps
+// the kernel's instruction footprint down.
+__device__ __noinline__ double sample_points(const double (*w_old)[3], double (*w_new)[3], const double *gbuf,
+                                             int num_levels, int level, const DevSystem &s, const LevelConst &lc,
+                                             int lane) {
   const int skip = 1 << (level + 1);
   const int nmid = (1 << num_levels) >> (level + 1);
-  warp_gaussians(rng, 3 * nmid, gbuf, lane);
-  __syncwarp();
-  const double levelTau = 0.5 * s.tau * skip;
-  const double sigma2 = (1.0 * s.lambda * levelTau);
-  const double sigma = sqrt(sigma2);
-  double lo = 0.0, ln = 0.0;
+  double d = 0.0;
   if (lane < nmid) {
     const int rel = lane * skip;
     const int mid = rel + (skip >> 1);
+    const double sigma = lc.sigma, hi2 = lc.half_inv;
     double rdiffOld[3], DeltaOld[3], rdiff[3], rbar[3], Delta[3];
     for (int i = 0; i < 3; i++) rdiffOld[i] = w_old[rel + skip][i] - w_old[rel][i];
     put_in_box(rdiffOld, s);
@@ -155,20 +222,21 @@ __device__ __forceinline__ double sample_level_warp(double (*w_old)[3], double (
     for (int i = 0; i < 3; i++) rbar[i] = w_new[rel][i] + 0.5 * rdiff[i];
     for (int i = 0; i < 3; i++) Delta[i] = gbuf[3 * lane + i] * sigma;
     put_in_box(Delta, s);
+    for (int i = 0; i < 3; i++) w_new[mid][i] = rbar[i] + Delta[i];
     // log of the image-summed Gaussian transition densities (BisectionStage.cc:241-256).
     // Without images, log(prod_d exp(-x_d)) = -sum_d x_d up to rounding while no
     // factor underflows; otherwise the reference's product is formed.
     bool direct = s.num_images == 0;
     double eo[3], en[3];
     for (int dim = 0; dim < 3; dim++) {
-      en[dim] = 0.5 * Delta[dim] * Delta[dim] / sigma2;
-      eo[dim] = 0.5 * DeltaOld[dim] * DeltaOld[dim] / sigma2;
+      en[dim] = Delta[dim] * Delta[dim] * hi2;
+      eo[dim] = DeltaOld[dim] * DeltaOld[dim] * hi2;
       direct = direct && en[dim] < 700.0 && eo[dim] < 700.0;
     }
     if (direct) {
-      lo = -(eo[0] + eo[1] + eo[2]);
-      ln = -(en[0] + en[1] + en[2]);
+      d = (en[0] + en[1] + en[2]) - (eo[0] + eo[1] + eo[2]);
     } else {
+      const double sigma2 = lc.sigma2;
       double GaussProd = 1.0, GaussProdOld = 1.0;
       for (int dim = 0; dim < 3; dim++) {
         double GaussSum = 0.0, GaussSumOld = 0.0;
@@ -181,28 +249,20 @@ __device__ __forceinline__ double sample_level_warp(double (*w_old)[3], double (
         GaussProd *= GaussSum;
         GaussProdOld *= GaussSumOld;
       }
-      lo = log(GaussProdOld);
-      ln = log(GaussProd);
+      d = log(GaussProdOld) - log(GaussProd);
     }
-    for (int i = 0; i < 3; i++) w_new[mid][i] = rbar[i] + Delta[i];
   }
-  lo = warp_sum_n(lo, nmid);
-  ln = warp_sum_n(ln, nmid);
+  d = warp_sum_n(d, nmid);
   __syncwarp();
-  return -ln + lo;
+  return d;
 }
-__device__ __noinline__ double sample_level_warp_outlined(double (*w_old)[3], double (*w_new)[3], double *gbuf,
-                                                          int num_levels, int level, const DevSystem &s,
-                                                          DevRandom &rng, int lane) {
-  return sample_level_warp(w_old, w_new, gbuf, num_levels, level, s, rng, lane);
-}
-// The level sampler: one out-of-line copy (OUTLINE: fewer cold instruction
-// lines per stage when a CTA runs many short jobs) or inlined at each call.
-template <bool OUTLINE>
-__device__ __forceinline__ double sample_level(double (*w_old)[3], double (*w_new)[3], double *gbuf, int num_levels,
-                                               int level, const DevSystem &s, DevRandom &rng, int lane) {
-  return OUTLINE ? sample_level_warp_outlined(w_old, w_new, gbuf, num_levels, level, s, rng, lane)
-                 : sample_level_warp(w_old, w_new, gbuf, num_levels, level, s, rng, lane);
+// The Gaussians of a level, then its points.
+__device__ __forceinline__ double sample_level(const double (*w_old)[3], double (*w_new)[3], double *gbuf,
+                                               int num_levels, int level, const DevSystem &s, const LevelConst *lc,
+                                               DevRandom &rng, int lane) {
+  warp_gaussians(rng, 3 * ((1 << num_levels) >> (level + 1)), gbuf, lane);
+  __syncwarp();
+  return sample_points(w_old, w_new, gbuf, num_levels, level, s, lc[level], lane);
 }
 
 }  // namespace
@@ -269,8 +329,12 @@ constexpr unsigned kTriTermBytes = 16u * kTriTermsPerWarp * sizeof(TriTerm);
 // [beg, beg + items) (item = link * np + partner index), each item evaluated
 // for the OLD and the NEW copy of the moved particle: 2 items (item, copy)
 // units.  Per pass every evaluating warp takes an even share of at most 96
-// consecutive units, three per lane (C2's 1022 level-0 units of a CTA in one
-// pass).  A lane forms its units' geometry
+// consecutive units, three per lane (1022 level-0 units of a CTA, 512 atoms on
+// 16 CTAs, in one pass), one after another: the unit's code once, and no
+// term held in registers over the next unit (unrolled with the terms listed at
+// the end: 5.77 ms for two rounds of 128 moves of 512 atoms, spilling; listed
+// as they come 5.24; one copy of the code 5.15; cells by magic-constant
+// rounding 4.84).  A lane forms its units' geometry
 // (DistDisp, q, z, s, the fit-region test, the cell) and adds the primitive
 // fallback of the terms outside the fit itself, from the potential's (y, d2y)
 // pairs in shared memory (pp; null: the global tables).  The terms inside the
@@ -297,20 +361,21 @@ __device__ __forceinline__ void tricubic_stage(const BisectionArgs &a, const dou
   for (int i = 0; i < lv; i++) beta *= 2.0;
   beta = 0.5 * beta;
   const int U = 2 * items;
-  const int P = (U + 3 * ethreads - 1) / (3 * ethreads);
-  const int cw = P > 0 ? (U + P * nw - 1) / (P * nw) : 0;  // <= 96
+  const int P = div_fast(U + 3 * ethreads - 1, 3 * ethreads);
+  const int cw = P > 0 ? div_fast(U + P * nw - 1, P * nw) : 0;  // <= 96
+  const float rnp = rcp_approx((float)np);
   for (int p = 0; p < P; p++) {
     const int ws = (p * nw + wi) * cw, we = min(U, ws + cw);
-    bool in[3];
-    TriTerm tt[3];
-#pragma unroll
+    int n = 0;  // terms listed
+#pragma unroll 1
     for (int s = 0; s < 3; s++) {
       const int u = ws + lane + 32 * s;
-      in[s] = false;
+      bool in = false;
+      TriTerm tt;
       if (u < we) {
         const int it = beg + (u >> 1);
         const int isn = u & 1;
-        const int link = it / np;
+        const int link = link_of(it, np, rnp);
         const int j = it - link * np;
         const int p2 = plist ? plist[j] : (j < ptcl ? j : j + 1);
         const int r0 = link * skip;
@@ -325,11 +390,11 @@ __device__ __forceinline__ void tricubic_stage(const BisectionArgs &a, const dou
         const LinkGeom<double> g = link_geom<double>(dA, dB);
         const TriPrep<double> pr = tricubic_prep<double>(t64, g.q, g.z, g.s2);
         if (pr.inside) {
-          in[s] = true;
-          tt[s].u[0] = pr.u[0];
-          tt[s].u[1] = pr.u[1];
-          tt[s].u[2] = pr.u[2];
-          tt[s].code = (pr.cell << 1) | isn;
+          in = true;
+          tt.u[0] = pr.u[0];
+          tt.u[1] = pr.u[1];
+          tt.u[2] = pr.u[2];
+          tt.code = (pr.cell << 1) | isn;
         } else {  // the primitive action 1/2 beta_l (V(r) + V(r'))
           const double v = pp ? pot_V_pairs(t64.pot_grid, pp, pr.r) + pot_V_pairs(t64.pot_grid, pp, pr.rp)
                               : pot_V(t64, pr.r) + pot_V(t64, pr.rp);
@@ -337,16 +402,16 @@ __device__ __forceinline__ void tricubic_stage(const BisectionArgs &a, const dou
         }
         if (SHADOW) (isn ? sn2 : so2) += tricubic_pa_mixed(t64, a.pa.t32, g.q, g.z, g.s2, lv).v;
       }
+      // listed at once: a term held over the next units costs the registers that
+      // keep their loads in flight
+      if (ws + 32 * s < we) {
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in) E[n + __popc(m & ((1u << lane) - 1u))] = tt;
+        n += __popc(m);
+      }
     }
-    // list the in-fit terms, then each team gathers every TPW-th of them
-    const unsigned m0 = __ballot_sync(0xffffffffu, in[0]), m1 = __ballot_sync(0xffffffffu, in[1]);
-    const unsigned m2 = __ballot_sync(0xffffffffu, in[2]);
-    const unsigned below = (1u << lane) - 1u;
-    const int n0 = __popc(m0), n1 = n0 + __popc(m1), n = n1 + __popc(m2);
-    if (in[0]) E[__popc(m0 & below)] = tt[0];
-    if (in[1]) E[n0 + __popc(m1 & below)] = tt[1];
-    if (in[2]) E[n1 + __popc(m2 & below)] = tt[2];
     __syncwarp();
+    // each team gathers every TPW-th of the terms
     for (int e = lane / TS; e < n; e += TPW) {
       const TriTerm T = E[e];
       ((T.code & 1) ? sn : so) += tricubic_team_part(F, t64, T.code >> 1, T.u, pt);
@@ -394,7 +459,7 @@ __device__ __forceinline__ StageSums stage_sums(const BisectionArgs &a, const do
     // a 2-lane team's (4.13e9 vs 3.91e9 C2 evals/s), so the mixed path keeps
     // one lane per term.
     const int total = np * nlinks;
-    const int chunk = (total + (int)CL - 1) / (int)CL;
+    const int chunk = div_fast(total + (int)CL - 1, (int)CL);
     const int beg = chunk * (int)rank;
     const int end = min(total, beg + chunk);
     if constexpr (!MIX)
@@ -403,96 +468,73 @@ __device__ __forceinline__ StageSums stage_sums(const BisectionArgs &a, const do
                              so2, sn2);
   } else if (lv == 0 || a.sr_higher) {  // ShortRangeClass::SingleAction over partners x links
     // partners: all others (plist null, np = N - 1) or the moved particle's
-    // neighbour list (np entries, ascending)
+    // neighbour list (np entries, ascending).  Item it is (link, j) =
+    // (it / np, it % np); the cluster's threads take the items in turn.
     const int total = np * nlinks;  // < 2^31: N <= 2^20, 2^L <= 64 (host-checked)
-    const int chunk = (total + (int)CL - 1) / (int)CL;
-    const int beg = chunk * (int)rank;
-    const int end = min(total, beg + chunk);
+    // Warps are numbered across the cluster first, so few items spread over its SMs.
+    const int NT = (int)CL * ethreads, gid = ((etid >> 5) * (int)CL + (int)rank) * 32 + (etid & 31);
     const double *path = a.path;
-    const int items = max(0, end - beg);
-    // Team size: when this CTA has fewer items than threads, T lanes share an
-    // item — the OLD and the NEW copy on different lanes and, for the tricubic
-    // fit, the four (x,y) node pairs split over the rest — which shortens the
-    // dependent chain of each lane.  T = 1 keeps one lane per item.
-    int T = 1;
-    const int tmax = KIND == PA_TRICUBIC ? 8 : 2;
-    while (T < tmax && items * T * 2 <= ethreads) T *= 2;
-    // When the items outnumber the threads but not twice over, a thread with
-    // a second item would evaluate four terms while most evaluate two; as
-    // (item, copy) units each thread evaluates at most ceil(2 items / threads)
-    // terms (the partner is then read once per copy).
-    const int per_item = 2 * ((items + ethreads - 1) / ethreads), per_unit = (2 * items + ethreads - 1) / ethreads;
-    if (T == 1 && per_unit < per_item) {
-      const int units = 2 * items;
-      for (int u0 = etid; u0 < units; u0 += 2 * ethreads) {
-        double a2[2][3], b2[2][3];
-        int r0s[2];
-        bool live[2], isn[2];
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          const int uu = u0 + u * ethreads;
-          live[u] = uu < units;
-          const int iu = live[u] ? uu : u0;
-          isn[u] = iu >= items;  // units [0, items) are the OLD copies, [items, 2 items) the NEW
-          const int it = beg + (isn[u] ? iu - items : iu);
-          const int link = it / np;
-          const int j = it - link * np;
-          const int p2 = plist ? plist[j] : (j < ptcl ? j : j + 1);
-          r0s[u] = link * skip;
-          const double *pa_ = path + ((size_t)(slice1 + r0s[u]) * N + p2) * 3;
-          const double *pb_ = path + ((size_t)(slice1 + r0s[u] + skip) * N + p2) * 3;
-          for (int i = 0; i < 3; i++) {
-            a2[u][i] = __ldcg(pa_ + i);
-            b2[u][i] = __ldcg(pb_ + i);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          if (!live[u]) continue;
-          const int r0 = r0s[u];
-          const double(*w)[3] = isn[u] ? w_new : w_old;
-          double dA[3], dB[3];
-          dist_disp(w[r0], a2[u], w[r0 + skip], b2[u], sys, dA, dB);
-          add_terms(link_geom<double>(dA, dB), isn[u], 0, 1);
-        }
+    const float rnp = rcp_approx((float)np);
+    // Positions of item (link, j)'s partner at the link's two slices.
+    auto partner = [&](int link, int j, int &r0, double a2[3], double b2[3]) {
+      const int p2 = plist ? plist[j] : (j < ptcl ? j : j + 1);
+      r0 = link * skip;
+      const double *pa_ = path + ((size_t)(slice1 + r0) * N + p2) * 3;
+      const double *pb_ = path + ((size_t)(slice1 + r0 + skip) * N + p2) * 3;
+      // L2-coherent loads: other CTAs write accepted windows during the launch.
+      for (int i = 0; i < 3; i++) {
+        a2[i] = __ldcg(pa_ + i);
+        b2[i] = __ldcg(pb_ + i);
       }
-    } else if (T == 1) {
-      // Two items per pass so a thread's partner and table loads overlap.
-      // Item it is (link, j) = (it / np, it % np); both pass items advance
-      // by the same stride, so (link, j) is carried instead of divided.
-      const int stride = 2 * ethreads;
-      const int qs = stride / np, rs = stride - qs * np;
+    };
+    auto one_copy = [&](const double (*w)[3], int r0, const double a2[3], const double b2[3], bool is_new, int part,
+                        int nparts) {
+      double dA[3], dB[3];
+      dist_disp(w[r0], a2, w[r0 + skip], b2, sys, dA, dB);
+      add_terms(link_geom<double>(dA, dB), is_new, part, nparts);
+    };
+    // (Single (item, copy) units for items between one and two a thread were
+    // slower at every shape tried: 188 atoms on 1 x 128 threads 8.7 against 8.0 ms.)
+    // Team size 2^lt: when the cluster has more threads than items, lanes share
+    // an item — the OLD and the NEW copy on different lanes and, for the tricubic
+    // fit, the four (x,y) node pairs split over the rest — which shortens the
+    // dependent chain of each lane.
+    constexpr int ltmax = KIND == PA_TRICUBIC ? 3 : 1;
+    int lt = 0;
+    while (lt < ltmax && (total << (lt + 1)) <= NT) lt++;
+    if (lt > 0) {
+      const int it = gid >> lt, member = gid & ((1 << lt) - 1);
+      if (it < total) {
+        const bool is_new = (member & 1) != 0;
+        double a2[3], b2[3];
+        int r0;
+        const int link = link_of(it, np, rnp);
+        partner(link, it - link * np, r0, a2, b2);
+        one_copy(is_new ? w_new : w_old, r0, a2, b2, is_new, member >> 1, 1 << (lt - 1));
+      }
+    } else {
+      // Two items per pass so a thread's partner and table loads overlap; both
+      // advance by the same stride, so (link, j) is carried.
+      const int stride = 2 * NT, qs = div_fast(stride, np), rs = stride - qs * np;
       int lk[2], jj[2];
 #pragma unroll
       for (int u = 0; u < 2; u++) {
-        const int it = beg + etid + u * ethreads;
-        lk[u] = it / np;
-        jj[u] = it - lk[u] * np;
+        lk[u] = div_fast(gid + u * NT, np);
+        jj[u] = gid + u * NT - lk[u] * np;
       }
-      for (int it0 = beg + etid; it0 < end; it0 += stride) {
+      for (int it0 = gid; it0 < total; it0 += stride) {
         double a2[2][3], b2[2][3];
         int r0s[2];
         bool live[2];
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-          const int it = it0 + u * ethreads;
-          live[u] = it < end;
-          const int link = live[u] ? lk[u] : lk[0];
-          const int j = live[u] ? jj[u] : jj[0];
-          const int p2 = plist ? plist[j] : (j < ptcl ? j : j + 1);
-          r0s[u] = link * skip;
-          const double *pa_ = path + ((size_t)(slice1 + r0s[u]) * N + p2) * 3;
-          const double *pb_ = path + ((size_t)(slice1 + r0s[u] + skip) * N + p2) * 3;
-          // L2-coherent loads: other CTAs write accepted windows during the launch.
-          for (int i = 0; i < 3; i++) {
-            a2[u][i] = __ldcg(pa_ + i);
-            b2[u][i] = __ldcg(pb_ + i);
-          }
+          live[u] = it0 + u * NT < total;
+          partner(live[u] ? lk[u] : lk[0], live[u] ? jj[u] : jj[0], r0s[u], a2[u], b2[u]);
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-          jj[u] += rs;
           lk[u] += qs;
+          jj[u] += rs;
           if (jj[u] >= np) {
             jj[u] -= np;
             lk[u]++;
@@ -501,31 +543,12 @@ __device__ __forceinline__ StageSums stage_sums(const BisectionArgs &a, const do
 #pragma unroll
         for (int u = 0; u < 2; u++) {
           if (!live[u]) continue;
-          const int r0 = r0s[u];
           double dAo[3], dBo[3], dAn[3], dBn[3];
-          dist_disp(w_old[r0], a2[u], w_old[r0 + skip], b2[u], sys, dAo, dBo);
-          dist_disp(w_new[r0], a2[u], w_new[r0 + skip], b2[u], sys, dAn, dBn);
+          dist_disp(w_old[r0s[u]], a2[u], w_old[r0s[u] + skip], b2[u], sys, dAo, dBo);
+          dist_disp(w_new[r0s[u]], a2[u], w_new[r0s[u] + skip], b2[u], sys, dAn, dBn);
           add_terms(link_geom<double>(dAo, dBo), false, 0, 1);
           add_terms(link_geom<double>(dAn, dBn), true, 0, 1);
         }
-      }
-    } else {
-      const int member = etid % T, team = etid / T, nteams = ethreads / T;
-      const bool is_new = (member & 1) != 0;
-      const int nparts = T >> 1, part = member >> 1;
-      const double(*w)[3] = is_new ? w_new : w_old;
-      for (int it = beg + team; it < end; it += nteams) {
-        const int link = it / np;
-        const int j = it - link * np;
-        const int p2 = plist ? plist[j] : (j < ptcl ? j : j + 1);
-        const int r0 = link * skip;
-        const double *pa_ = path + ((size_t)(slice1 + r0) * N + p2) * 3;
-        const double *pb_ = path + ((size_t)(slice1 + r0 + skip) * N + p2) * 3;
-        const double a2[3] = {__ldcg(pa_), __ldcg(pa_ + 1), __ldcg(pa_ + 2)};
-        const double b2[3] = {__ldcg(pb_), __ldcg(pb_ + 1), __ldcg(pb_ + 2)};
-        double dA[3], dB[3];
-        dist_disp(w[r0], a2, w[r0 + skip], b2, sys, dA, dB);
-        add_terms(link_geom<double>(dA, dB), is_new, part, nparts);
       }
     }
   }
@@ -536,11 +559,9 @@ __device__ __forceinline__ StageSums stage_sums(const BisectionArgs &a, const do
     // Madelung and background terms are the same in both and cancel in dS.
     const int nk = a.nk;
     const int total = (span + 1) * nk;
-    const int chunk = (total + (int)CL - 1) / (int)CL;
-    const int beg = chunk * (int)rank;
-    const int end = min(total, beg + chunk);
-    for (int it = beg + etid; it < end; it += ethreads) {
-      const int rel = it / nk, k = it - rel * nk;
+    const float rnk = rcp_approx((float)nk);
+    for (int it = ((etid >> 5) * (int)CL + (int)rank) * 32 + (etid & 31); it < total; it += (int)CL * ethreads) {
+      const int rel = link_of(it, nk, rnk), k = it - rel * nk;
       const double f = (rel == 0 || rel == span) ? 0.5 : 1.0;
       const double2 ro = __ldcg(&a.rhok[(size_t)(slice1 + rel) * nk + k]);
       const double *kv = a.kvec + 3 * k;
@@ -580,13 +601,12 @@ __device__ __forceinline__ StageSums stage_sums(const BisectionArgs &a, const do
 // while the other warps evaluate the pair terms, so no evaluating thread
 // starts its partner loads late.  The sums are identical in every lane.
 __device__ __forceinline__ double2 kinetic_sums(const double (*w_old)[3], const double (*w_new)[3], int num_levels,
-                                                int lv, const DevSystem &sys, int lane) {
+                                                int lv, const DevSystem &sys, const LevelConst *lc, int lane) {
   double so = 0.0, sn = 0.0;
   if (sys.lambda != 0.0) {
     const int skip = 1 << lv;
     const int nlinks = (1 << num_levels) >> lv;
-    const double levelTau = sys.tau * (1 << lv);
-    const double F = 1.0 / (4.0 * sys.lambda * levelTau);
+    const double F = lc[lv].kinF;
     for (int k = lane; k < nlinks; k += 32) {
       double vo[3], vn[3];
       for (int i = 0; i < 3; i++) {
@@ -680,10 +700,20 @@ constexpr int kNbrStage = 1024;
 // the two shadow sums.
 constexpr int kRed = 5;
 
+// Counters of a move and of a job, kept in shared memory:
+// in registers every thread of the block would hold them.
+struct MoveCounts {
+  unsigned long long stages, pairs, flips, reevals;
+};
+struct JobCounts {
+  MoveCounts c;
+  unsigned long long moves, accepted, redone;
+};
+
 // Shared state of one CTA while it runs a job.
 struct KernelShared {
   double win_old[2][kMaxWindow][3], win_new[2][kMaxWindow][3];
-  double gbuf[2][3 * 32];
+  double gbuf[3 * 32], gbuf_next[3];  // unit Gaussians of a level; of the next move's top level
   double sh_red[16][kRed];  // per warp: S_old, S_new, the mixed bound, the shadows
   double xchg[2][kMaxCluster][kRed];
   double s_logsr[kMaxLevels], s_logu[kMaxLevels];
@@ -697,7 +727,7 @@ struct KernelShared {
   // speculated next one), whether a NEW position of the current stage lies
   // outside it, and whether this job evaluates all partners from now on
   double4 s_cb, s_next_cb;
-  int s_far, s_next_far, s_allpairs;
+  int s_far, s_far1, s_next_far, s_allpairs;
   // concurrent proposals: the stream position at the start of this slot's
   // move (restored when the move is redone), the outcome every slot of the
   // window published for the in-order commit, and the commit's verdict
@@ -710,7 +740,16 @@ struct KernelShared {
   // Stage reduction across the cluster: per parity an mbarrier that completes
   // when every CTA's partials have landed in xchg[parity] (st.async).
   uint64_t red_bar[2];
+  LevelConst lc[kMaxLevels];
+  DevSystem sys;  // for the out-of-line sampler (a reference into the kernel's parameters would put them on the stack)
+  // The move's record as the lead thread fills it (dS, bounds, re-evaluations);
+  // written out and cleared by the sampler warp at the end of the move.
+  pimc_move_record rec;
+  JobCounts tot;
+  MoveCounts mv;  // concurrent proposals: counted when the move is kept
 };
+constexpr int kRecWords = (int)(sizeof(pimc_move_record) / sizeof(int));
+static_assert(kRecWords <= 64, "two words a lane");
 // Tries of the wait for a stage reduction's partials before PIMC_E_CAP.
 constexpr int kRedWaitCap = 1 << 24;
 
@@ -787,15 +826,24 @@ struct Group {
   int tid;       // thread index within the group
   int size;      // threads in the group, a multiple of 32
   unsigned bar;  // named barrier id
+  // Producer / consumer barriers of a stage, `n` threads each: the evaluating
+  // warps' sums for warp 0 (ebar), the samplers' results for warp 0 (sbar).
+  unsigned ebar, sbar;
   __device__ __forceinline__ void sync() const {
     asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(size) : "memory");
+  }
+  static __device__ __forceinline__ void arrive(unsigned id, int n) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+  }
+  static __device__ __forceinline__ void wait(unsigned id, int n) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
   }
 };
 
 // The moves of one job — one chain, or one window of a chain — on this CTA
 // (cluster rank `rank` of `CL`).  `phase` is the parity of the table-staging
 // mbarrier `bar`, flipped once per staging.
-template <int KIND, typename R, bool SHADOW, bool OUTLINE, bool PROP = false>
+template <int KIND, typename R, bool SHADOW, bool PROP = false>
 __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsigned rank, unsigned CL,
                         cg::cluster_group &cluster, const Group &G, unsigned char *dyn, unsigned dyn_cap,
                         KernelShared &S, uint64_t *bar_ptr, unsigned &phase, const RngTab &tab_mem,
@@ -830,16 +878,24 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
   // move may start from a window another slot is about to write)
   const int specwarp = (nwarps >= 4 && !prop) ? nwarps - 2 : -1;
   const int ethreads = (nwarps - (specwarp >= 0 ? 2 : 1)) * 32;  // evaluating threads: warps below the samplers
-  // The moved particle's kinetic links: with 8 or more evaluating warps the
+  // The moved particle's kinetic links: with 4 or more evaluating warps the
   // last of them sums them after its pair terms (the item split leaves it the
   // fewest), so the level sampler's warp only samples; otherwise the sampler.
-  const int kinwarp = (ethreads >> 5) >= 8 ? (ethreads >> 5) - 1 : -1;
+  // (On the sampler of an 8-warp block they ended 1500 cycles after the terms.)
+  const int kinwarp = (ethreads >> 5) >= 4 ? (ethreads >> 5) - 1 : -1;
   const bool evaluator = tid < ethreads;
+  // Rows of sh_red a stage's reduction adds: the evaluating warps', and the
+  // sampler's where it sums the kinetic links (before it samples).
+  const int nred = (ethreads >> 5) + (kinwarp < 0 ? 1 : 0);
+  const int sthreads = specwarp >= 0 ? 96 : 64;  // samplers and warp 0
   const DevSystem &sys = a.sys;
   const int N = sys.N;
   const int L = a.num_levels;
   const int span = 1 << L;
   const bool lead = (erank == 0 && tid == 0);
+  // Counters of the job: the sampler warp, which is off a stage's critical path
+  // (re-evaluations and flips, which are rare, by the lead thread).
+  const bool counter = erank == 0 && warp == sampler && lane == 0;
 
   // ---- stage 1-D tables into shared memory (bulk TMA) ----
   // DavidPA: the diagonal columns of every level, each diag_stride pairs
@@ -942,8 +998,11 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
     S.s_allpairs = 0;
     S.tab = tab_mem;
     S.tab.W = 0;  // filled below
+    S.tot = JobCounts{};
   }
-  unsigned long long moves = 0, accepted = 0, stages = 0, pair_evals = 0, flips = 0, redone = 0, reevals = 0;
+  if (tid < L) S.lc[tid] = level_const(sys, tid);
+  if (tid == 0) S.sys = sys;
+  if (tid < kRecWords) reinterpret_cast<int *>(&S.rec)[tid] = 0;
   int status = 0;
   double *path = a.path;
   unsigned xc = 0;  // exchange parity counter
@@ -969,9 +1028,12 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
   }
   if (staged && CL > 1) cluster.sync();  // every CTA has read xchg[1]
   // Stage reductions over a cluster: each CTA's red_bar[p] expects the
-  // partials of every CTA (kRed doubles each) for its next use; the first
+  // partials of every CTA (NV doubles each) for its next use; the first
   // uses are posted before the cluster barrier, so before any peer can send.
-  const unsigned red_bytes = CL * kRed * (unsigned)sizeof(double);
+  // Values a stage's reduction carries: the two sums; mixed: the bound, and in a
+  // re-evaluation the previous stage's two sums; with the shadow all of them.
+  constexpr int NV = SHADOW ? kRed : std::is_same<R, float>::value ? 4 : 2;
+  const unsigned red_bytes = CL * NV * (unsigned)sizeof(double);
   unsigned rph = 0;  // phase parity of red_bar[0] (bit 0) and red_bar[1] (bit 1)
   if (ECL > 1) {
     if (tid == 0) {
@@ -998,18 +1060,19 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
   // position at the start of the move.
   const int P = prop ? a.proposals : 1;
   int pstep = 0, pfirst = 0;
+  int bstep = 0;  // this move's step of its block
 
   for (int m = 0; prop ? pstep < a.steps_per_block : m < total_moves; m++) {
-    const int blk = prop ? 0 : m / a.steps_per_block, step = prop ? pstep : m - blk * a.steps_per_block;
+    const int step = prop ? pstep : bstep;
     const bool active = !prop || (int)rank >= pfirst;
     // this move's work: counted at once, or with proposals when the move is kept
-    unsigned long long mv_stages = 0, mv_pairs = 0, mv_flips = 0, mv_reevals = 0;
-    unsigned long long &c_stages = PROP ? mv_stages : stages, &c_pairs = PROP ? mv_pairs : pair_evals,
-                       &c_flips = PROP ? mv_flips : flips, &c_reevals = PROP ? mv_reevals : reevals;
+    if (PROP && counter) S.mv = MoveCounts{};
+    MoveCounts &cnt_ = PROP ? S.mv : S.tot.c;
     bool acc_all = true;
     int move_far = 0;  // some stage of this move sampled outside the moved particle's sphere
     int mptcl = 0;     // the moved particle
-    pimc_move_record rec;
+    int passed = 0;
+    pimc_move_record &rec = S.rec;
     if (active) {
       if (!have_next) {
         // ChooseTimeSlices (BisectionBlock.cc:362-374), ChooseParticle (NoPermuteClass.cc:61-68)
@@ -1035,7 +1098,7 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
         G.sync();
         if (warp == sampler) {
           DevRandom rng = rng_from(s_rng, seed, stream, &S.tab);
-          const double lsr = sample_level<OUTLINE>(win_old[cur], win_new[cur], gbuf[0], L, L - 1, sys, rng, lane);
+          const double lsr = sample_level(win_old[cur], win_new[cur], gbuf, L, L - 1, S.sys, S.lc, rng, lane);
           const double lu = rng.LocalLog();
           int far = 0;
           double4 cb = make_double4(0.0, 0.0, 0.0, 0.0);
@@ -1059,7 +1122,7 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
       const int ptcl = s_ctl[1];
       mptcl = ptcl;
       const bool more = m + 1 < total_moves;
-      const bool next_new_block = !a.concurrent && ((m + 1) % a.steps_per_block == 0);
+      const bool next_new_block = !a.concurrent && bstep + 1 == a.steps_per_block;
       double(*w_old)[3] = win_old[cur];
       double(*w_new)[3] = win_new[cur];
       // Neighbour lists: the moved particle's list (fixed for the launch) in
@@ -1081,17 +1144,6 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
       double prevDS = 0.0, prevDS_s = 0.0, prevE = 0.0;
       int prev_np = 0;
       const int *prev_plist = nullptr;
-      int passed = 0;
-      if (lead) {
-        rec.slice1 = slice1;
-        rec.ptcl = ptcl;
-        for (int i = 0; i < 8; i++) {
-          rec.dS[i] = rec.dS_shadow[i] = 0.0;
-          rec.dS_bound[i] = 0.0f;
-        }
-        rec.reevaluated = 0;
-        rec.pad = 0;
-      }
       int si = 0;
       for (int level = L - 1; level >= 0; level--, si++) {
         // ---- LocalStageClass::Attempt (StageClass.cc:49-95) ----
@@ -1121,32 +1173,42 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
           const StageSums v = stage_sums<KIND, R, SHADOW>(a, w_old, w_new, diag_smem ? diag_smem + level * st : nullptr,
                                                           diag_smem_s ? diag_smem_s + level * sts : nullptr, level,
                                                           slice1, ptcl, erank, ECL, tid, ethreads, plist, np, tq);
-          double r0 = warp_sum(v.so), r1 = warp_sum(v.sn);
-          const double r2 = warp_sum(v.eb);
-          double r3 = SHADOW ? warp_sum(v.so2) : 0.0, r4 = SHADOW ? warp_sum(v.sn2) : 0.0;
+          // sums of the warp: S_old in the lower half, S_new in the upper
+          double r0 = warp_sum_pair(v.so, v.sn, lane);
+          const double r2 = std::is_same<R, float>::value ? warp_sum(v.eb) : 0.0;
+          double r3 = SHADOW ? warp_sum_pair(v.so2, v.sn2, lane) : 0.0;
           if (warp == kinwarp && erank == 0) {
             // the moved particle's kinetic links, once per evaluation group
-            const double2 k = kinetic_sums(w_old, w_new, L, level, sys, lane);
-            r0 += k.x;
-            r1 += k.y;
-            r3 += k.x;
-            r4 += k.y;
+            const double2 k = kinetic_sums(w_old, w_new, L, level, sys, S.lc, lane);
+            r0 += lane < 16 ? k.x : k.y;
+            if (SHADOW) r3 += lane < 16 ? k.x : k.y;
           }
-          if (lane == 0) {
-            sh_red[warp][0] = r0;
-            sh_red[warp][1] = r1;
-            sh_red[warp][2] = r2;
-            sh_red[warp][3] = r3;
-            sh_red[warp][4] = r4;
+          if ((lane & 15) == 0) {
+            sh_red[warp][lane >> 4] = r0;
+            if (NV > 2 && lane == 0) sh_red[warp][2] = r2;
+            if (SHADOW) sh_red[warp][3 + (lane >> 4)] = r3;
           }
+          __syncwarp();
+          if (warp != 0) Group::arrive(G.ebar, nred * 32);
         } else {
+          if (warp == sampler && kinwarp < 0) {
+            // the moved particle's kinetic links, once per evaluation group
+            const double2 k = erank == 0 ? kinetic_sums(w_old, w_new, L, level, sys, S.lc, lane)
+                                         : make_double2(0.0, 0.0);
+            if (lane < kRed) sh_red[nred - 1][lane] = lane == 2 ? 0.0 : (lane == 0 || lane == 3) ? k.x : k.y;
+            __syncwarp();
+            Group::arrive(G.ebar, nred * 32);
+          }
           if (warp == sampler && level > 0) {
             // speculative sampling of the next level (BisectionStage::Sample of stage level-1)
             DevRandom spec = rng_from(s_rng, seed, stream, &S.tab);
-            const double lsr = sample_level<OUTLINE>(w_old, w_new, gbuf[0], L, level - 1, sys, spec, lane);
+            const double lsr = sample_level(w_old, w_new, gbuf, L, level - 1, S.sys, S.lc, spec, lane);
             const double lu = spec.LocalLog();
+            // neighbour lists: whether the next stage's NEW positions leave the sphere
+            const int far = a.nbr_on ? window_outside(w_new, span, S.s_cb, sys, lane) : 0;
             __syncwarp();
             if (lane == 0) {
+              S.s_far1 = far;
               s_logsr[level - 1] = lsr;
               s_logu[level - 1] = lu;
               rng_store(s_spec1, spec);
@@ -1166,7 +1228,9 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
               for (int i = 0; i < 3; i++) wo[rel][i] = wn[rel][i] = __ldcg(q + i);
             }
             __syncwarp();
-            const double lsr = sample_level<OUTLINE>(wo, wn, gbuf[1], L, L - 1, sys, spec, lane);
+            warp_gaussians(spec, 3, S.gbuf_next, lane);
+            __syncwarp();
+            const double lsr = sample_points(wo, wn, S.gbuf_next, L, L - 1, S.sys, S.lc[L - 1], lane);
             const double lu = spec.LocalLog();
             int far = 0;
             if (a.nbr_on) {
@@ -1184,49 +1248,39 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
               rng_store(s_spec2, spec);
             }
           }
-          if (lane < kRed) sh_red[warp][lane] = 0.0;
-          if (warp == sampler && erank == 0 && kinwarp < 0) {
-            // the moved particle's kinetic links, once per evaluation group
-            const double2 k = kinetic_sums(w_old, w_new, L, level, sys, lane);
-            __syncwarp();
-            if (lane == 0) {
-              sh_red[warp][0] = k.x;
-              sh_red[warp][1] = k.y;
-              sh_red[warp][3] = k.x;
-              sh_red[warp][4] = k.y;
-            }
+          if (counter) {
+            // Counted as the reference performs them: OLD + NEW of the stage's links.
+            if (level == 0 || a.sr_higher) cnt_.pairs += 2ull * (unsigned long long)np * (span >> level);
+            cnt_.stages++;
           }
+          __syncwarp();
+          Group::arrive(G.sbar, sthreads);
         }
-        // Counted as the reference performs them: OLD + NEW of the stage's links.
-        if (lead && (level == 0 || a.sr_higher)) c_pairs += 2ull * (unsigned long long)np * (span >> level);
-        G.sync();
         // ---- reduce: warps -> CTA (warp 0) -> cluster (DSMEM, rank order) ----
         // The sums are bitwise the same in every CTA of the cluster, so every
         // CTA takes the same decision (and the same re-evaluation request).
-        auto reduce = [&]() -> double {
+        // Two values at a time, a warp's (then a rank's) partial a lane: values
+        // v and v + 1 in the warp's halves, added by a butterfly over 16 lanes.
+        auto reduce = [&](double out[NV + 1]) {
           const int par = xc & 1;
-          xc++;
-          double v = 0.0;
-          if (warp != 0) return v;
-          if (lane < kRed) {
-            // all loads first, then a fixed pairwise tree (16 warps at most)
-            double t[16];
+          const int half = lane >> 4, w = lane & 15;
+          Group::wait(G.ebar, nred * 32);
+          double x[(NV + 1) / 2];
 #pragma unroll
-            for (int w = 0; w < 16; w++) t[w] = w < nwarps ? sh_red[w][lane] : 0.0;
+          for (int v = 0; v < NV; v += 2) x[v / 2] = w < nred && v + half < NV ? sh_red[w][v + half] : 0.0;
 #pragma unroll
-            for (int h = 8; h > 0; h >>= 1)
+          for (int o = 8; o > 0; o >>= 1)
 #pragma unroll
-              for (int w = 0; w < h; w++) t[w] += t[w + h];
-            v = t[0];
-            if (ECL > 1) {
-              // this CTA's partials into xchg[par][rank] of every CTA of the cluster
-              const unsigned dst = smem_addr(&xchg[par][rank][lane]), bar = smem_addr(&S.red_bar[par]);
-              for (unsigned r = 0; r < CL; r++) st_async_f64(mapa_u32(dst, r), v, mapa_u32(bar, r));
-            } else {
-              xchg[par][0][lane] = v;
-            }
-          }
+            for (int v = 0; v < NV; v += 2) x[v / 2] += __shfl_xor_sync(0xffffffffu, x[v / 2], o);
           if (ECL > 1) {
+            // this CTA's partials into xchg[par][rank] of every CTA of the cluster,
+            // lane w (and w + 16) to CTA w
+            const unsigned to = w < (int)CL ? w : 0;
+            const unsigned dst = mapa_u32(smem_addr(&xchg[par][rank][half]), to);
+            const unsigned bar = mapa_u32(smem_addr(&S.red_bar[par]), to);
+#pragma unroll
+            for (int v = 0; v < NV; v += 2)
+              if (w < (int)CL && v + half < NV) st_async_f64(dst + v * (unsigned)sizeof(double), x[v / 2], bar);
             // Bounded wait for every CTA's partials.  A peer sends to this
             // buffer again only for the reduction after next, which needs
             // this CTA's next partials, so the next use is posted now.
@@ -1234,20 +1288,21 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
             for (int it = 0; it < kRedWaitCap && !ok; it++) ok = mbar_try_wait_cluster(&S.red_bar[par], (rph >> par) & 1u);
             rph ^= 1u << par;
             if (!ok) status = PIMC_E_CAP;
+#pragma unroll
+            for (int v = 0; v < NV; v += 2) x[v / 2] = w < (int)CL && v + half < NV ? xchg[par][w][v + half] : 0.0;
             __syncwarp();
             if (lane == 0) mbar_expect_tx(&S.red_bar[par], red_bytes);
-          } else {
-            __syncwarp();
-          }
-          v = 0.0;
-          if (lane < kRed) {  // rank order, loads first
-            double t[kMaxCluster];
 #pragma unroll
-            for (int r = 0; r < kMaxCluster; r++) t[r] = r < (int)ECL ? xchg[par][r][lane] : 0.0;
+            for (int o = 8; o > 0; o >>= 1)
 #pragma unroll
-            for (int r = 0; r < kMaxCluster; r++) v += t[r];
+              for (int v = 0; v < NV; v += 2) x[v / 2] += __shfl_xor_sync(0xffffffffu, x[v / 2], o);
           }
-          return v;
+          xc++;
+#pragma unroll
+          for (int v = 0; v < NV; v += 2) {
+            out[v] = __shfl_sync(0xffffffffu, x[v / 2], 0);
+            out[v + 1] = __shfl_sync(0xffffffffu, x[v / 2], 16);
+          }
         };
         // ---- Metropolis test, identical in every CTA (warp 0) ----
         // exact: so/sn are the FP64 sums (the FP64 path, or the mixed path's
@@ -1288,7 +1343,7 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
           if (SHADOW) {
             const double dss = sn2 - so2;
             const bool other = (logsr - dss + prevDS_s) >= logu;
-            if (other != toAccept && lead) c_flips++;
+            if (other != toAccept && lead) cnt_.flips++;
             prevDS_s = dss;
             if (lead && si < 8) rec.dS_shadow[si] = dss;
           }
@@ -1300,9 +1355,6 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
           }
           // commit the stream position the outcome selects
           const bool ends = !toAccept || level == 0 || status != 0;
-          // neighbour lists: whether the next stage's NEW positions (the level
-          // sampled speculatively into w_new) leave the moved particle's sphere
-          const int far_next = (a.nbr_on && !ends) ? window_outside(w_new, span, S.s_cb, sys, lane) : 0;
           if (lane == 0) {
             S.s_need[0] = 0;
             s_ctl[2] = toAccept ? 1 : 0;
@@ -1310,7 +1362,7 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
             int nv = 0;
             if (!ends) {
               s_rng = s_spec1;
-              S.s_far = far_next;
+              S.s_far = S.s_far1;  // of the level sampled speculatively into w_new
             } else if (status == 0 && more && specwarp >= 0 && !(toAccept && s_next[2] == ptcl)) {
               s_rng = s_spec2;
               s_ctl[0] = s_next[1];
@@ -1324,14 +1376,12 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
             s_next[0] = nv;
           }
         };
-        {
-          const double v = reduce();
-          if (warp == 0) {
-            const double so = __shfl_sync(0xffffffffu, v, 0), sn = __shfl_sync(0xffffffffu, v, 1);
-            const double eb = __shfl_sync(0xffffffffu, v, 2);
-            const double so2 = __shfl_sync(0xffffffffu, v, 3), sn2 = __shfl_sync(0xffffffffu, v, 4);
-            decide(so, sn, std::is_same<R, float>::value ? eb : 0.0, so2, sn2, !std::is_same<R, float>::value);
-          }
+        if (warp == 0) {
+          double r[NV + 1];
+          reduce(r);
+          Group::wait(G.sbar, sthreads);  // the samplers' speculation, which the decision commits
+          decide(r[0], r[1], std::is_same<R, float>::value ? r[2] : 0.0, SHADOW ? r[SHADOW ? 3 : 0] : 0.0,
+                 SHADOW ? r[SHADOW ? 4 : 0] : 0.0, !std::is_same<R, float>::value);
         }
         G.sync();
         if (std::is_same<R, float>::value && S.s_need[0]) {
@@ -1343,50 +1393,41 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
           if (evaluator) {
             const double4 v = stage_sums_reeval<KIND>(a, w_old, w_new, level, slice1, ptcl, erank, ECL, tid, ethreads,
                                                       plist, np, need_prev, prev_plist, prev_np, tq);
-            double r0 = warp_sum(v.x), r1 = warp_sum(v.y), r2 = warp_sum(v.z), r3 = warp_sum(v.w);
+            double r0 = warp_sum_pair(v.x, v.y, lane), r2 = warp_sum_pair(v.z, v.w, lane);
             if (warp == kinwarp && erank == 0) {  // the kinetic links, as in the first pass
-              const double2 k = kinetic_sums(w_old, w_new, L, level, sys, lane);
-              const double2 kp = need_prev ? kinetic_sums(w_old, w_new, L, level + 1, sys, lane)
-                                           : make_double2(0.0, 0.0);
-              r0 += k.x;
-              r1 += k.y;
-              r2 += kp.x;
-              r3 += kp.y;
-            }
-            if (lane == 0) {
-              sh_red[warp][0] = r0;
-              sh_red[warp][1] = r1;
-              sh_red[warp][2] = r2;
-              sh_red[warp][3] = r3;
-              sh_red[warp][4] = 0.0;
-            }
-          } else {
-            if (lane < kRed) sh_red[warp][lane] = 0.0;
-            if (warp == sampler && erank == 0 && kinwarp < 0) {  // the kinetic links, as in the first pass
-              const double2 k = kinetic_sums(w_old, w_new, L, level, sys, lane);
-              const double2 kp = need_prev ? kinetic_sums(w_old, w_new, L, level + 1, sys, lane)
-                                           : make_double2(0.0, 0.0);
-              __syncwarp();
-              if (lane == 0) {
-                sh_red[warp][0] = k.x;
-                sh_red[warp][1] = k.y;
-                sh_red[warp][2] = kp.x;
-                sh_red[warp][3] = kp.y;
+              const double2 k = kinetic_sums(w_old, w_new, L, level, sys, S.lc, lane);
+              r0 += lane < 16 ? k.x : k.y;
+              if (need_prev) {
+                const double2 kp = kinetic_sums(w_old, w_new, L, level + 1, sys, S.lc, lane);
+                r2 += lane < 16 ? kp.x : kp.y;
               }
             }
+            if ((lane & 15) == 0) {
+              sh_red[warp][lane >> 4] = r0;
+              if (NV > 2) sh_red[warp][2 + (lane >> 4)] = r2;
+              if (SHADOW) sh_red[warp][4] = 0.0;
+            }
+            __syncwarp();
+            if (warp != 0) Group::arrive(G.ebar, nred * 32);
+          } else if (warp == sampler && kinwarp < 0) {  // the kinetic links, as in the first pass
+            const double2 k = erank == 0 ? kinetic_sums(w_old, w_new, L, level, sys, S.lc, lane)
+                                         : make_double2(0.0, 0.0);
+            const double2 kp = erank == 0 && need_prev ? kinetic_sums(w_old, w_new, L, level + 1, sys, S.lc, lane)
+                                                       : make_double2(0.0, 0.0);
+            if (lane < kRed)
+              sh_red[nred - 1][lane] = lane == 0 ? k.x : lane == 1 ? k.y : lane == 2 ? kp.x : lane == 3 ? kp.y : 0.0;
+            __syncwarp();
+            Group::arrive(G.ebar, nred * 32);
           }
-          if (lead) c_reevals++;
-          G.sync();
-          const double v = reduce();
+          if (lead) cnt_.reevals++;
           if (warp == 0) {
-            const double so = __shfl_sync(0xffffffffu, v, 0), sn = __shfl_sync(0xffffffffu, v, 1);
-            const double pso = __shfl_sync(0xffffffffu, v, 2), psn = __shfl_sync(0xffffffffu, v, 3);
-            if (need_prev) prevDS = psn - pso;
-            decide(so, sn, 0.0, so, sn, true);
+            double r[NV + 1];
+            reduce(r);
+            if (need_prev) prevDS = r[NV > 2 ? 3 : 0] - r[NV > 2 ? 2 : 0];
+            decide(r[0], r[1], 0.0, r[0], r[1], true);
           }
           G.sync();
         }
-        if (tid == 0) c_stages++;
         prev_np = np;
         prev_plist = plist;
         if (!s_ctl[2] || s_ctl[3]) {
@@ -1396,14 +1437,47 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
         passed++;
       }
       have_next = s_next[0] != 0;
-      if (lead) {
-        rec.accepted = acc_all ? 1 : 0;
-        rec.stages_passed = passed;
-      }
     }  // active
+    const int move_status = s_ctl[3];
+    // The move's record, by the sampler warp: its words (and S.rec cleared for
+    // the next move) in take_record, the trace slot `at` in put_record.
+    const int rec_slice1 = slice1;
+    int rec_w[2] = {0, 0};
+    auto take_record = [&]() {
+      if (erank != 0 || warp != sampler) return;
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const int i = lane + 32 * k;
+        if (i >= kRecWords) break;
+        int *w = reinterpret_cast<int *>(&S.rec) + i;
+        rec_w[k] = i == 0 ? rec_slice1 : i == 1 ? mptcl : i == 2 ? (acc_all ? 1 : 0) : i == 3 ? passed : *w;
+        *w = 0;
+      }
+    };
+    auto put_record = [&](long long at) {
+      if (erank != 0 || warp != sampler || !a.trace) return;
+      int *t = reinterpret_cast<int *>(a.trace + a.trace_offset + at);
+#pragma unroll
+      for (int k = 0; k < 2; k++)
+        if (lane + 32 * k < kRecWords) t[lane + 32 * k] = rec_w[k];
+    };
     // ---- AcceptCopy (PathClass.cc:797-863); a rejected move left HBM untouched ----
     // The moved particle's window (and, with long range, the window's rho_k)
     // by this CTA's threads.
+    // The window's rows by threads [0, n), t this one's index: with concurrent
+    // windows only the interior slices, since the end slices are shared with the
+    // neighbouring windows and never move, and boxing them here would race with
+    // the neighbour's read of the same slice.
+    auto write_window = [&](int t, int n) {
+      for (int rel = (a.concurrent ? 1 : 0) + t; rel <= (a.concurrent ? span - 1 : span); rel += n) {
+        double v[3] = {win_new[cur][rel][0], win_new[cur][rel][1], win_new[cur][rel][2]};
+        put_in_box_fast(v, sys);
+        double *q = path + ((size_t)(slice1 + rel) * N + mptcl) * 3;
+        q[0] = v[0];
+        q[1] = v[1];
+        q[2] = v[2];
+      }
+    };
     auto accept_copy = [&](bool write_path) {
       if (a.use_lr) {
         // AcceptCopy of rho_k (PathClass.cc:797-863): the NEW rho_k of the
@@ -1415,36 +1489,25 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
         // windows, and their update is rounding only).
         const int lo = a.concurrent ? 1 : 0, hi = a.concurrent ? span - 1 : span;
         const int nk = a.nk, total = (hi - lo + 1) * nk;
+        const float rnk = rcp_approx((float)nk);
         for (int it = (int)erank * G.size + tid; it < total; it += (int)ECL * G.size) {
-          const int rel = lo + it / nk, k = it - (it / nk) * nk;
+          const int row = link_of(it, nk, rnk), rel = lo + row, k = it - row * nk;
           double2 *p2 = &a.rhok[(size_t)(slice1 + rel) * nk + k];
           const double2 rn = rho_new_k<double>(__ldcg(p2), a.kvec + 3 * k, win_new[cur][rel], win_old[cur][rel]);
           __stcg(p2, rn);
         }
       }
-      // With concurrent windows only the interior slices: the end slices are
-      // shared with the neighbouring windows and never move, and boxing them
-      // here would race with the neighbour's read of the same slice.
-      if (write_path)
-        for (int rel = (a.concurrent ? 1 : 0) + tid; rel <= (a.concurrent ? span - 1 : span); rel += G.size) {
-          double v[3] = {win_new[cur][rel][0], win_new[cur][rel][1], win_new[cur][rel][2]};
-          put_in_box_fast(v, sys);
-          double *q = path + ((size_t)(slice1 + rel) * N + mptcl) * 3;
-          q[0] = v[0];
-          q[1] = v[1];
-          q[2] = v[2];
-        }
+      if (write_path) write_window(tid, G.size);
     };
-    auto count_move = [&](long long at) {  // by the lead thread
-      moves++;
-      if (acc_all) accepted++;
+    auto count_move = [&]() {  // by the counting thread
+      S.tot.moves++;
+      if (acc_all) S.tot.accepted++;
       if (PROP) {
-        stages += mv_stages;
-        pair_evals += mv_pairs;
-        flips += mv_flips;
-        reevals += mv_reevals;
+        S.tot.c.stages += S.mv.stages;
+        S.tot.c.pairs += S.mv.pairs;
+        S.tot.c.flips += S.mv.flips;
+        S.tot.c.reevals += S.mv.reevals;
       }
-      if (a.trace) a.trace[a.trace_offset + at] = rec;
     };
     if (!PROP) {
       if (acc_all && move_far) {
@@ -1453,25 +1516,29 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
         if (tid == 0) S.s_allpairs = 1;
         if (lead) atomicExch(a.nbr_dirty, 1);
       }
-      if (acc_all) {
-        accept_copy(rank == 0);
-        if (CL > 1)
-          cluster.sync();
-        else
-          G.sync();
-      }
-      if (lead)
-        count_move(a.concurrent ? (long long)window * a.steps_per_block + step
-                                : (long long)blk * a.steps_per_block + step);
-      if (s_ctl[3] != 0) break;
+      // On a cluster the accepted window is written by CTA 0's sampler warp alone,
+      // and only it (and with rho_k everyone) arrives at the cluster barrier with
+      // release: the flush of its few rows is a thousand cycles that the other
+      // warps spend on the bookkeeping and then wait out.
+      const bool meet = acc_all && CL > 1;
+      const bool writer = meet && rank == 0 && warp == sampler;
+      if (acc_all) accept_copy(CL == 1);
+      if (writer) write_window(lane, 32);
+      take_record();
+      if (counter) count_move();
       if (have_next) cur ^= 1;
       G.sync();  // every thread has read s_ctl / s_next before the next move rewrites them
+      if (meet) cluster_arrive(writer || a.use_lr);
+      put_record(a.concurrent ? (long long)window * a.steps_per_block + m : (long long)m);
+      if (++bstep == a.steps_per_block) bstep = 0;
+      if (meet) cluster_wait();
+      if (move_status != 0) break;
     } else {
       // ---- in-order commit of the pass ----
       // Every slot publishes its outcome to every CTA of the window: accepted,
       // particle, whether it left its sphere, status.
       if (tid == 0) {
-        const int4 pub = active ? make_int4(acc_all ? 1 : 0, mptcl, move_far, s_ctl[3]) : make_int4(0, -1, 0, 0);
+        const int4 pub = active ? make_int4(acc_all ? 1 : 0, mptcl, move_far, move_status) : make_int4(0, -1, 0, 0);
         for (unsigned r = 0; r < CL; r++) cluster.map_shared_rank(&S.s_pub[rank], r)[0] = pub;
         S.s_redo_local = 0;
       }
@@ -1516,11 +1583,14 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
       const int nf = S.s_commit[0];
       if (active && (int)rank < nf) {
         if (acc_all) accept_copy(true);
-        if (lead) count_move(((long long)window * a.steps_per_block + step) * P + rank);
+        if (counter) count_move();
+        take_record();
+        put_record(((long long)window * a.steps_per_block + step) * P + rank);
       } else if (active) {
+        take_record();
         if (tid == 0) {
           s_rng = S.s_rng0;  // the redo draws from the move's first number again
-          redone++;
+          S.tot.redone++;
         }
       }
       if (S.s_commit[2]) {
@@ -1546,13 +1616,13 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
     cs->nlocal = s_rng.n;
     cs->one_left = s_rng.one_left;
     cs->x2 = s_rng.x2;
-    cs->moves += moves;
-    cs->accepted += accepted;
-    cs->stages += stages;
-    cs->pair_evals += pair_evals;
-    cs->flips += flips;
-    cs->redone += redone;
-    cs->reevals += reevals;
+    cs->moves += S.tot.moves;
+    cs->accepted += S.tot.accepted;
+    cs->stages += S.tot.c.stages;
+    cs->pair_evals += S.tot.c.pairs;
+    cs->flips += S.tot.c.flips;
+    cs->redone += S.tot.redone;
+    cs->reevals += S.tot.c.reevals;
     if (status) cs->status = status;
   }
   if (CL > 1) cluster.sync();
@@ -1583,12 +1653,12 @@ __global__ void __launch_bounds__(512, 1) bisection_kernel(BisectionArgs a) {
   __syncthreads();
   unsigned phase = 0;
   ChainState *cs = a.chains + (a.concurrent ? (PROP ? (int)rank * kMaxWindows + window : window) : 0);
-  const Group G = {(int)threadIdx.x, (int)blockDim.x, 0u};
+  const Group G = {(int)threadIdx.x, (int)blockDim.x, 0u, 1u, 2u};
   unsigned dyn_size;
   asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_size));
   const RngTab tab = store.part<2>(0, 2);
-  run_job<KIND, R, SHADOW, false, PROP>(a, cs, window, rank, CL, cluster, G, dyn, dyn_size, S, &s_bar, phase, tab,
-                                        s_nbr);
+  run_job<KIND, R, SHADOW, PROP>(a, cs, window, rank, CL, cluster, G, dyn, dyn_size, S, &s_bar, phase, tab,
+                                  s_nbr);
 }
 
 // Many independent chains in one persistent launch (the reference's clone
@@ -1628,7 +1698,8 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(BatchArgs b) {
   unsigned phase = 0;
   for (int guard = 0; guard < 2 * b.n_chains + 2 * kSlots + 2; guard++) {
     const int gsize = (int)blockDim.x >> k;
-    const Group G = {(int)threadIdx.x - p * gsize, gsize, (1u << k) + (unsigned)p};
+    const unsigned quarter = (unsigned)(p << (kMaxSplit - k));  // ids 1-7 the groups' own, 8-15 by quarter of the CTA
+    const Group G = {(int)threadIdx.x - p * gsize, gsize, (1u << k) + (unsigned)p, 8u + quarter, 12u + quarter};
     const int slot = p << (b.max_split - k);
     if (c < 0) {
       if (G.tid == 0) s_chain[slot] = (int)atomicAdd(b.queue, 1u);
@@ -1663,7 +1734,7 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(BatchArgs b) {
     }
     G.sync();
     const RngTab tab = store.part<kSlots>(p << (kMaxSplit - k), 1 << (kMaxSplit - k));
-    run_job<KIND, R, SHADOW, true>(job, job.chains, 0, 0, 1, cluster, G, dyn + (size_t)slot * b.dyn_per_slot,
+    run_job<KIND, R, SHADOW>(job, job.chains, 0, 0, 1, cluster, G, dyn + (size_t)slot * b.dyn_per_slot,
                              b.dyn_per_slot, S[slot], &s_bar[slot], phase, tab);
     c = -1;
   }

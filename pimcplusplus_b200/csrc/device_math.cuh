@@ -322,9 +322,9 @@ __device__ __forceinline__ void dist_disp(const double a1[3], const double a2[3]
   for (int i = 0; i < 3; i++) {
     double da = a2[i] - a1[i];
     double db = b2[i] - b1[i];
-    double n = -rint(rmul(da, s.boxinv[i]));
+    double n = -round_even_magic(rmul(da, s.boxinv[i]));
     da = radd(da, rmul(n, s.box[i]));
-    double m = rint(rmul(rsub(da, db), s.boxinv[i]));
+    double m = round_even_magic(rmul(rsub(da, db), s.boxinv[i]));
     db = radd(db, rmul(m, s.box[i]));
     dA[i] = da;
     dB[i] = db;
@@ -335,8 +335,10 @@ __device__ __forceinline__ void dist_disp(const double a1[3], const double a2[3]
 __device__ __forceinline__ void put_in_box(double v[3], const DevSystem &s) {
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    double n = -floor(radd(rmul(v[i], s.boxinv[i]), 0.5));
-    v[i] = radd(v[i], rmul(n, s.box[i]));
+    const double t = radd(rmul(v[i], s.boxinv[i]), 0.5);
+    double n = round_even_magic(t);  // floor(t), as above on the FP64 pipe
+    if (n > t) n -= 1.0;
+    v[i] = radd(v[i], rmul(-n, s.box[i]));
   }
 }
 // PathClass::PutInBoxFast (PathClass.cc:1389-1407)
@@ -676,11 +678,12 @@ __device__ __forceinline__ TriPrep<R> tricubic_prep(const DTricubic<double> &t, 
   int i3[3];
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    int i = reverse_map(*g[d], x[d]);
-    i = max(0, i);
-    i = min(i, g[d]->n - 2);
-    i3[d] = i;
-    p.u[d] = (R)((x[d] - grid_x(*g[d], i)) * g[d]->deltainv);
+    // the cell as integers held in FP64 (spline_cell): conversions to and from
+    // integers are a quarter-rate detour on every term's chain
+    const double rm = round_even_magic(rsub(rmul(rsub(x[d], g[d]->start), g[d]->deltainv), 0.5));
+    const double lowf = fmin(fmax(rm, 0.0), (double)(g[d]->n - 2));
+    i3[d] = int_of_integral(lowf);
+    p.u[d] = (R)((x[d] - radd(g[d]->start, rmul(lowf, g[d]->delta))) * g[d]->deltainv);
   }
   p.cell = (i3[0] * t.ny + i3[1]) * t.nt + i3[2];
   p.r = q + 0.5 * z;
