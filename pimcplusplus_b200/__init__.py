@@ -230,6 +230,18 @@ def _iptr(a):
     return a.ctypes.data_as(_ip)
 
 
+def _int_list(values):
+    """(C int array, length) of a particle list.  A short list or tuple of plain
+    ints goes straight into a ctypes array: numpy and ndarray.ctypes cost several
+    us, a third of an action call; everything else takes numpy's conversion."""
+    if type(values) in (list, tuple):
+        n = len(values)
+        if n <= 64 and all(type(v) is int and -0x80000000 <= v <= 0x7fffffff for v in values):
+            return (_i * n)(*values), n
+    a = np.ascontiguousarray(values, dtype=np.int32)
+    return _iptr(a), len(a)
+
+
 def read_dm(path, desired_tau):
     """Host-only: the DavidPA tables of a squarer .dm file as the library reads them.
 
@@ -370,10 +382,11 @@ class PathData:
 
     # ---- actions ----
     def single_action(self, action, copy, slice1, slice2, active, level, precision=FP64):
-        a = np.ascontiguousarray(active, dtype=np.int32)
+        a, n = _int_list(active)
         out = C.c_double()
-        self._check(_lib.pimc_single_action(self.h, action, copy, slice1, slice2, _iptr(a), len(a), level,
-                                            precision, C.byref(out)), "single_action")
+        rc = _lib.pimc_single_action(self.h, action, copy, slice1, slice2, a, n, level, precision, C.byref(out))
+        if rc:
+            self._check(rc, "single_action")
         return out.value
 
     def d_dbeta(self, action, slice1, slice2, level=0):
@@ -382,12 +395,12 @@ class PathData:
         return out.value
 
     def AcceptCopy(self, slice1, slice2, active):
-        a = np.ascontiguousarray(active, dtype=np.int32)
-        self._check(_lib.pimc_accept_copy(self.h, slice1, slice2, _iptr(a), len(a)), "accept_copy")
+        a, n = _int_list(active)
+        self._check(_lib.pimc_accept_copy(self.h, slice1, slice2, a, n), "accept_copy")
 
     def RejectCopy(self, slice1, slice2, active):
-        a = np.ascontiguousarray(active, dtype=np.int32)
-        self._check(_lib.pimc_reject_copy(self.h, slice1, slice2, _iptr(a), len(a)), "reject_copy")
+        a, n = _int_list(active)
+        self._check(_lib.pimc_reject_copy(self.h, slice1, slice2, a, n), "reject_copy")
 
     def synchronize(self):
         self._check(_lib.pimc_synchronize(self.h), "synchronize")
@@ -425,8 +438,8 @@ class PathData:
         self._check(_lib.pimc_calc_rhok(self.h), "calc_rhok")
 
     def update_rhok(self, slice1, slice2, active, level):
-        a = np.ascontiguousarray(active, dtype=np.int32)
-        self._check(_lib.pimc_update_rhok(self.h, slice1, slice2, _iptr(a), len(a), level), "update_rhok")
+        a, n = _int_list(active)
+        self._check(_lib.pimc_update_rhok(self.h, slice1, slice2, a, n, level), "update_rhok")
 
     def get_rhok(self, copy=OLDMODE):
         out = np.empty((self.S, self.num_k, 2))
@@ -571,7 +584,8 @@ class BisectionBlock:
 
     def MakeMoves(self, n_blocks, trace=True):
         st = BisectionStats()
-        rec = (np.zeros(n_blocks * self.windows * self.steps_per_block * self.proposals, dtype=MOVE_RECORD)
+        # every record is written by the call
+        rec = (np.empty(n_blocks * self.windows * self.steps_per_block * self.proposals, dtype=MOVE_RECORD)
                if trace else None)
         ptr = rec.ctypes.data_as(_p) if trace else None
         self.PathData._check(_lib.pimc_run_bisection(self.PathData.h, n_blocks, ptr, C.byref(st)), "run_bisection")
@@ -648,7 +662,7 @@ class BatchChains:
 
     def run(self, n_blocks, trace=False):
         st = BisectionStats()
-        rec = np.zeros(self.n * n_blocks * self.steps, dtype=MOVE_RECORD) if trace else None
+        rec = np.empty(self.n * n_blocks * self.steps, dtype=MOVE_RECORD) if trace else None
         ptr = rec.ctypes.data_as(_p) if trace else None
         self._check(_lib.pimc_batch_run(self.h, n_blocks, ptr, C.byref(st)), "batch_run")
         if trace:

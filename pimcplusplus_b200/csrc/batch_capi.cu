@@ -458,6 +458,22 @@ int pimc_batch_autotune(pimc_batch *b, int n_blocks, int *threads_out, int *ctas
   return PIMC_OK;
 }
 
+// Counters of one chain, or of all (-1).
+static void sum_states(const std::vector<ChainState> &cs, int chain, pimc_bisection_stats *stats) {
+  std::memset(stats, 0, sizeof(*stats));
+  for (int i = 0; i < (int)cs.size(); i++) {
+    if (chain >= 0 && i != chain) continue;
+    const ChainState &c = cs[i];
+    stats->moves += (int64_t)c.moves;
+    stats->accepted += (int64_t)c.accepted;
+    stats->stages_attempted += (int64_t)c.stages;
+    stats->pair_evals += (int64_t)c.pair_evals;
+    stats->flips += (int64_t)c.flips;
+    stats->reevaluated += (int64_t)c.reevals;
+    if (c.status && !stats->status) stats->status = c.status;
+  }
+}
+
 int pimc_batch_run(pimc_batch *b, int n_blocks, pimc_move_record *trace, pimc_bisection_stats *stats) {
   if (!b || n_blocks < 0) return PIMC_E_ARG;
   BCK(cudaSetDevice(b->device));
@@ -475,11 +491,12 @@ int pimc_batch_run(pimc_batch *b, int n_blocks, pimc_move_record *trace, pimc_bi
   if (trace) BCK(cudaMemsetAsync(b->d_trace, 0, nrec * sizeof(pimc_move_record), b->stream));
   int rc = batch_launch(b, n_blocks, trace ? b->d_trace : nullptr, per_chain);
   if (rc) return rc;
+  std::vector<ChainState> cs(b->n_chains);
+  BCK(cudaMemcpyAsync(cs.data(), b->d_chains, cs.size() * sizeof(ChainState), cudaMemcpyDeviceToHost, b->stream));
   if (trace) BCK(cudaMemcpyAsync(trace, b->d_trace, nrec * sizeof(pimc_move_record), cudaMemcpyDeviceToHost, b->stream));
   BCK(cudaStreamSynchronize(b->stream));
   pimc_bisection_stats st;
-  rc = pimc_batch_get_stats(b, -1, &st);
-  if (rc) return rc;
+  sum_states(cs, -1, &st);
   if (stats) *stats = st;
   if (st.status) return bfail(b, st.status, std::string("device status: ") + pimc_status_string(st.status));
   return PIMC_OK;
@@ -491,18 +508,7 @@ int pimc_batch_get_stats(pimc_batch *b, int chain, pimc_bisection_stats *stats) 
   std::vector<ChainState> cs(b->n_chains);
   BCK(cudaMemcpyAsync(cs.data(), b->d_chains, cs.size() * sizeof(ChainState), cudaMemcpyDeviceToHost, b->stream));
   BCK(cudaStreamSynchronize(b->stream));
-  std::memset(stats, 0, sizeof(*stats));
-  for (int i = 0; i < b->n_chains; i++) {
-    if (chain >= 0 && i != chain) continue;
-    const ChainState &c = cs[i];
-    stats->moves += (int64_t)c.moves;
-    stats->accepted += (int64_t)c.accepted;
-    stats->stages_attempted += (int64_t)c.stages;
-    stats->pair_evals += (int64_t)c.pair_evals;
-    stats->flips += (int64_t)c.flips;
-    stats->reevaluated += (int64_t)c.reevals;
-    if (c.status && !stats->status) stats->status = c.status;
-  }
+  sum_states(cs, chain, stats);
   return PIMC_OK;
 }
 

@@ -259,7 +259,9 @@ int pimc_create(const pimc_system_desc *d, pimc_context **out) {
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_partials, kPartialSlots * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_counter, sizeof(unsigned int));
   if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned int), ctx->stream);
-  if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_out, 4 * sizeof(double));
+  if (e == cudaSuccess)  // one pinned page: the scalars, then the states of a sequential chain or of every window
+    e = cudaMallocHost(&ctx->h_out, 4 * sizeof(double) + kMaxWindows * sizeof(ChainState));
+  if (e == cudaSuccess) ctx->h_chain = reinterpret_cast<ChainState *>(ctx->h_out + 4);
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_bounds, pair_path_bounds_bytes(s.N, s.S));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_chain, kMaxChainStates * sizeof(ChainState));
   if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_chain, 0, kMaxChainStates * sizeof(ChainState), ctx->stream);
@@ -293,6 +295,7 @@ int pimc_destroy(pimc_context *ctx) {
   cudaFree(ctx->d_dulong_k);
   cudaFree(ctx->d_yk);
   cudaFree(ctx->d_gofr);
+  if (ctx->h_gofr) cudaFreeHost(ctx->h_gofr);
   cudaFree(ctx->d_kvec);
   cudaFree(ctx->d_nbr_cb);
   cudaFree(ctx->d_nbr_cnt);
@@ -771,8 +774,40 @@ int pimc_bisection_setup(pimc_context *ctx, const pimc_bisection_desc *d) {
     c.status = 0;
   }
   CK(copy_sync(ctx, ctx->d_chain, cs.data(), cs.size() * sizeof(ChainState)));
+  ctx->states_used = d->schedule == PIMC_SCHEDULE_SEQUENTIAL ? 1
+                     : d->schedule == PIMC_SCHEDULE_WINDOWS  ? kMaxWindows
+                                                             : kMaxChainStates;
   ctx->bis_ready = true;
   return PIMC_OK;
+}
+
+// The move counters.  A set-up clears them all and a run touches the states of
+// its schedule only, so those are read back (all 1024 after a checkpoint was
+// read): into pinned memory where they fit.  enqueue_states before the stream's
+// synchronisation, sum_states after it.
+static int enqueue_states(pimc_context *ctx, std::vector<ChainState> &all) {
+  ChainState *dst = ctx->h_chain;
+  if (ctx->states_used > kMaxWindows) {
+    all.resize(ctx->states_used);
+    dst = all.data();
+  }
+  CK(cudaMemcpyAsync(dst, ctx->d_chain, ctx->states_used * sizeof(ChainState), cudaMemcpyDeviceToHost, ctx->stream));
+  return PIMC_OK;
+}
+static void sum_states(const pimc_context *ctx, const std::vector<ChainState> &all, pimc_bisection_stats *stats) {
+  const ChainState *cs = all.empty() ? ctx->h_chain : all.data();
+  std::memset(stats, 0, sizeof(*stats));
+  for (int i = 0; i < ctx->states_used; i++) {
+    const ChainState &c = cs[i];
+    stats->moves += (int64_t)c.moves;
+    stats->accepted += (int64_t)c.accepted;
+    stats->stages_attempted += (int64_t)c.stages;
+    stats->pair_evals += (int64_t)c.pair_evals;
+    stats->flips += (int64_t)c.flips;
+    stats->redone += (int64_t)c.redone;
+    stats->reevaluated += (int64_t)c.reevals;
+    if (c.status && !stats->status) stats->status = c.status;
+  }
 }
 
 int pimc_rng_seed(pimc_context *ctx, uint64_t seed) {
@@ -894,12 +929,13 @@ int pimc_run_bisection(pimc_context *ctx, int n_blocks, pimc_move_record *trace,
   if (ctx->bis.use_longrange)
     CK(cudaMemcpyAsync(ctx->d_rhok[1], ctx->d_rhok[0], (size_t)ctx->sys.S * ctx->num_k * sizeof(double2),
                        cudaMemcpyDeviceToDevice, ctx->stream));
+  std::vector<ChainState> all;
+  if ((rc = enqueue_states(ctx, all))) return rc;
   if (trace && nrec)
     CK(cudaMemcpyAsync(trace, ctx->d_trace, nrec * sizeof(pimc_move_record), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   pimc_bisection_stats st;
-  rc = pimc_bisection_get_stats(ctx, &st);
-  if (rc) return rc;
+  sum_states(ctx, all, &st);
   if (stats) *stats = st;
   if (st.status) {
     // The status belongs to this call: clear it so that the next call on the
@@ -916,20 +952,10 @@ int pimc_run_bisection(pimc_context *ctx, int n_blocks, pimc_move_record *trace,
 int pimc_bisection_get_stats(pimc_context *ctx, pimc_bisection_stats *stats) {
   if (!ctx || !stats) return PIMC_E_ARG;
   CK(cudaSetDevice(ctx->device));
-  std::vector<ChainState> cs(kMaxChainStates);
-  CK(cudaMemcpyAsync(cs.data(), ctx->d_chain, cs.size() * sizeof(ChainState), cudaMemcpyDeviceToHost, ctx->stream));
+  std::vector<ChainState> all;
+  if (int rc = enqueue_states(ctx, all)) return rc;
   CK(cudaStreamSynchronize(ctx->stream));
-  std::memset(stats, 0, sizeof(*stats));
-  for (const auto &c : cs) {
-    stats->moves += (int64_t)c.moves;
-    stats->accepted += (int64_t)c.accepted;
-    stats->stages_attempted += (int64_t)c.stages;
-    stats->pair_evals += (int64_t)c.pair_evals;
-    stats->flips += (int64_t)c.flips;
-    stats->redone += (int64_t)c.redone;
-    stats->reevaluated += (int64_t)c.reevals;
-    if (c.status && !stats->status) stats->status = c.status;
-  }
+  sum_states(ctx, all, stats);
   return PIMC_OK;
 }
 
@@ -1237,6 +1263,9 @@ int pimc_gofr_setup(pimc_context *ctx, double start, double end, int num_points)
   CK(cudaSetDevice(ctx->device));
   cudaFree(ctx->d_gofr);
   ctx->d_gofr = nullptr;
+  if (ctx->h_gofr) cudaFreeHost(ctx->h_gofr);
+  ctx->h_gofr = nullptr;
+  CK(cudaMallocHost(&ctx->h_gofr, (size_t)(num_points - 1) * sizeof(unsigned long long)));
   CK(cudaMalloc(&ctx->d_gofr, (size_t)(num_points - 1) * sizeof(unsigned long long)));
   CK(cudaMemsetAsync(ctx->d_gofr, 0, (size_t)(num_points - 1) * sizeof(unsigned long long), ctx->stream));
   ctx->gofr_points = num_points;
@@ -1264,8 +1293,8 @@ int pimc_gofr_get(pimc_context *ctx, uint64_t *histogram, double *gofr, long lon
   if (!ctx->d_gofr) return fail(ctx, PIMC_E_STATE, "pimc_gofr_setup not called");
   CK(cudaSetDevice(ctx->device));
   const int nb = ctx->gofr_points - 1;
-  std::vector<unsigned long long> h(nb);
-  CK(cudaMemcpyAsync(h.data(), ctx->d_gofr, nb * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
+  const unsigned long long *h = ctx->h_gofr;
+  CK(cudaMemcpyAsync(ctx->h_gofr, ctx->d_gofr, nb * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   if (histogram)
     for (int i = 0; i < nb; i++) histogram[i] = h[i];

@@ -247,6 +247,7 @@ int pimc_checkpoint_read(pimc_context *ctx, const char *filename) {
   IOCK(cudaMemcpyAsync(ctx->d_path[1], paths.data() + elems, elems * sizeof(double), cudaMemcpyHostToDevice,
                        ctx->stream));
   IOCK(cudaMemcpyAsync(ctx->d_chain, cs.data(), cs.size() * sizeof(ChainState), cudaMemcpyHostToDevice, ctx->stream));
+  ctx->states_used = kMaxChainStates;  // whatever schedule wrote it
   ctx->rounds = counters[0];
   ctx->seed = counters[1];
   ctx->shift_draws = counters[2];

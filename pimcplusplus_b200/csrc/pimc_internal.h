@@ -182,12 +182,14 @@ struct pimc_context {
   double *d_partials = nullptr;
   unsigned int *d_counter = nullptr;
   double *h_out = nullptr;  // pinned, written by the reduction kernels
+  pimc::ChainState *h_chain = nullptr;  // behind h_out: kMaxWindows states
   float4 *d_bounds = nullptr;  // bounding spheres of the pair sums (pair_path.cu)
   int *d_active = nullptr;
   // bisection
   pimc_bisection_desc bis{};
   bool bis_ready = false;
-  pimc::ChainState *d_chain = nullptr;  // kMaxWindows states
+  pimc::ChainState *d_chain = nullptr;  // kMaxChainStates states
+  int states_used = pimc::kMaxChainStates;  // the first ones, which can hold counts
   unsigned long long rounds = 0;         // concurrent-window rounds run so far
   uint64_t seed = 0;                     // the key pimc_rng_seed set
   unsigned long long shift_draws = 0;    // ShiftMove draws taken from stream 3
@@ -217,7 +219,7 @@ struct pimc_context {
   double *d_yk = nullptr;
   bool yk_ready = false;
   // pair correlation accumulator (PairCorrelationClass)
-  unsigned long long *d_gofr = nullptr;
+  unsigned long long *d_gofr = nullptr, *h_gofr = nullptr;  // device bins; pinned copy
   int gofr_points = 0;
   double gofr_start = 0, gofr_end = 0, gofr_delta = 0, gofr_deltainv = 0;
   long long gofr_counts = 0;
