@@ -47,7 +47,8 @@ struct BisectionArgs {
 };
 
 // Neighbour lists for the device moves (neighbors.cu): rebuilt from the
-// current path when *dirty is set, then *dirty cleared.
+// current path when dirty[0] is set, which is then cleared (dirty[1]: a counter,
+// zero between launches).
 cudaError_t launch_nbr_rebuild(cudaStream_t st, const double *path, const DevSystem &sys, double range, double skin,
                                int kmax, double4 *cb, int *cnt, int *idx, int *dirty);
 

@@ -759,7 +759,8 @@ int pimc_bisection_setup(pimc_context *ctx, const pimc_bisection_desc *d) {
     CK(cudaMalloc(&ctx->d_nbr_cb, (size_t)ctx->sys.N * sizeof(double4)));
     CK(cudaMalloc(&ctx->d_nbr_cnt, (size_t)ctx->sys.N * sizeof(int)));
     CK(cudaMalloc(&ctx->d_nbr_idx, (size_t)ctx->sys.N * kmax * sizeof(int)));
-    CK(cudaMalloc(&ctx->d_nbr_dirty, sizeof(int)));
+    CK(cudaMalloc(&ctx->d_nbr_dirty, 2 * sizeof(int)));
+    CK(cudaMemsetAsync(ctx->d_nbr_dirty, 0, 2 * sizeof(int), ctx->stream));
     CK(cudaMemsetAsync(ctx->d_nbr_dirty, 0xff, sizeof(int), ctx->stream));
     ctx->nbr_kmax = kmax;
     ctx->nbr_range = ctx->pa.d64.grid.end;  // the table is zero from its last point on
