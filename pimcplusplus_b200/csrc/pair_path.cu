@@ -20,7 +20,7 @@
 // Measured as pimc_energy, against one thread per (pair, link) that decoded its
 // indices with 64-bit divisions and evaluated both ends of every link, and a
 // second such pass for V: N = 4096, M = 256, range 0.11 of the box 73.7 -> 0.57
-// ms; N = 512, M = 128, tricubic 1042 -> 688 us; N = 128, M = 64, Coulomb
+// ms; N = 512, M = 128, tricubic 1042 -> 625 us; N = 128, M = 64, Coulomb
 // (both passes) 34 -> 22 us.  FP64 operations and their latencies bound it.
 #include <cuda_runtime.h>
 
@@ -33,9 +33,10 @@ namespace pimc {
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kWarps = kThreads / 32;
 constexpr int kMaxTile = 64;
+// Threads a block (tricubic, N = 512: 128 threads 625 us, 256 608; N = 37: 32.6, 34.3)
+template <int KIND>
+constexpr int kThreadsOf = KIND == PA_TRICUBIC ? 128 : 256;
 
 struct PairPathArgs {
   const double *path;
@@ -117,21 +118,61 @@ __device__ __forceinline__ void displacement(const double *a, const double *b, c
   }
 }
 
-// One in-fit tricubic term listed for the warp's lane teams.
-struct PathTerm {
+// One in-fit tricubic term listed for the warp's lane teams: its in-cell
+// coordinates and its cell.  (With the Hermite bases in the list, 112 bytes a
+// term, the team's lanes save work but the L1 left for the node table misses:
+// no gain; a third more blocks an SM: 842 us against 648.)
+struct __align__(16) PathTerm {
   double u[3];
-  int cell, pad;
+  int cell;
 };
+
+// One lane's part of a listed term: components 4 (pt & 1) .. + 3 of node
+// iz + (pt >> 1) of the cell's four (x, y) node pairs (as tricubic_team_part,
+// with the sums over y taken first).
+__device__ __forceinline__ double team_part(const double *F, const DTricubic<double> &t, const PathTerm &P, int pt) {
+  const size_t sy = (size_t)t.nt * 8, sx = (size_t)t.ny * sy;
+  const int nz = pt >> 1, hi = pt & 1;
+  const double *p = F + (size_t)P.cell * 8 + nz * 8 + hi * 4;
+  double v[4][4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) ld4_nc(p + (k >> 1) * sx + (k & 1) * sy, v[k]);
+  double a[4], b[4], c[4];
+  hermite4(P.u[0], t.qg.delta, a);
+  hermite4(P.u[1], t.yg.delta, b);
+  hermite4(P.u[2], t.tg.delta, c);
+  // (F, Fx, Fy, Fz) weigh (A0 B0 Cv, A1 B0 Cv, A0 B1 Cv, A0 B0 Cd), (Fxy, Fxz,
+  // Fyz, Fxyz) weigh (A1 B1 Cv, A1 B0 Cd, A0 B1 Cd, A1 B1 Cd)
+  const double Cv = nz ? c[1] : c[0], Cd = nz ? c[3] : c[2], Ce = hi ? Cd : Cv;
+  double s = 0.0, e = 0.0;
+#pragma unroll
+  for (int dx = 0; dx < 2; dx++) {
+    double x = 0.0, y = 0.0, z = 0.0;
+#pragma unroll
+    for (int dy = 0; dy < 2; dy++) {
+      const double *w = v[2 * dx + dy];
+      x += (hi ? b[2 + dy] : b[dy]) * (Cv * w[0] + Cd * w[3]);
+      y += b[dy] * w[1];
+      z += b[2 + dy] * w[2];
+    }
+    s += (hi ? a[2 + dx] : a[dx]) * x;
+    e += a[2 + dx] * y + a[dx] * z;
+  }
+  return s + Ce * e;
+}
 
 // KIND's d_dBeta over links and, with DO_V, V over slices 0 .. nlinks (weight
 // 1/2 at both ends; slice1 = 0 and skip = 1 then).  out[0] = d_dBeta, out[1] = V.
 template <int KIND, bool DO_V>
-__global__ void __launch_bounds__(kThreads, KIND == PA_TRICUBIC ? 2 : 3)
+__global__ void __launch_bounds__(kThreadsOf<KIND>, KIND == PA_TRICUBIC ? 4 : 3)
     pair_path_kernel(const __grid_constant__ PairPathArgs a, double2 *partials, unsigned int *counter, double *out) {
+  constexpr int kThreads = kThreadsOf<KIND>, kWarps = kThreads / 32;
+  constexpr int kStep = KIND == PA_TRICUBIC ? 4 : 1;  // links between two gathers: their terms fill the teams' rounds
   __shared__ float4 s_bi[kMaxTile], s_bj[kMaxTile];
   __shared__ unsigned short s_list[kMaxTile * kMaxTile];
   __shared__ int s_cnt[kWarps + 1];
-  __shared__ PathTerm s_terms[KIND == PA_TRICUBIC ? kWarps * 64 : 1];
+  __shared__ PathTerm s_terms[KIND == PA_TRICUBIC ? kWarps * 32 * kStep : 1];
+  PathTerm *const E = s_terms + (KIND == PA_TRICUBIC ? (threadIdx.x >> 5) * 32 * kStep : 0);
   __shared__ double sh[2][kWarps];
   __shared__ int s_last;
   const DevSystem &sys = a.sys;
@@ -255,14 +296,13 @@ __global__ void __launch_bounds__(kThreads, KIND == PA_TRICUBIC ? 2 : 3)
       double ra = sqrt(dA[0] * dA[0] + dA[1] * dA[1] + dA[2] * dA[2]);
       SliceVal va = {0.0, 0.0}, vb = {0.0, 0.0};
       if (live && (KIND != PA_TRICUBIC || DO_V)) va = slice_value<KIND, DO_V>(a.pa, tb, ra);
-      constexpr int kStep = KIND == PA_TRICUBIC ? 2 : 1;
       for (int l = l0; l < l0 + len; l += kStep) {
-        PathTerm tt[kStep];
-        bool in[kStep];
-#pragma unroll
+        int listed = 0;
+#pragma unroll 1
         for (int k = 0; k < kStep; k++) {
-          in[k] = false;
-          if (!live || l + k >= l1) continue;
+          bool in = false;
+          PathTerm tt;
+          if (live && l + k < l1) {
           pi += row;
           pj += row;
           displacement(pi, pj, sys, raw, dB);
@@ -296,12 +336,10 @@ __global__ void __launch_bounds__(kThreads, KIND == PA_TRICUBIC ? 2 : 3)
             du += a.pa.c64.z1z2 / (0.5 * (ra + rl)) - 0.5 * (va.f + fl);
           } else {
             const TriPrep<double> pr = tricubic_prep<double>(a.pa.t64, 0.5 * (ra + rl), ra - rl, s2);
-            in[k] = pr.inside;
+            in = pr.inside;
             if (pr.inside) {
-              tt[k].u[0] = pr.u[0];
-              tt[k].u[1] = pr.u[1];
-              tt[k].u[2] = pr.u[2];
-              tt[k].cell = pr.cell;
+              for (int x = 0; x < 3; x++) tt.u[x] = pr.u[x];
+              tt.cell = pr.cell;
             } else if (DO_V) {
               du += 0.5 * (va.f + fl);
             } else {
@@ -313,22 +351,19 @@ __global__ void __launch_bounds__(kThreads, KIND == PA_TRICUBIC ? 2 : 3)
           for (int x = 0; x < 3; x++) dA[x] = dB[x];
           ra = rb;
           va = vb;
+          }
+          if (KIND == PA_TRICUBIC) {
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (in) E[listed + __popc(m & ((1u << lane) - 1u))] = tt;
+            listed += __popc(m);
+          }
         }
         if (KIND == PA_TRICUBIC) {
           // The in-fit terms of the warp's step, gathered by teams of four
-          // lanes (tricubic_team_part): a cell's node pair is one 128-byte
-          // line a team, against a line a lane.
-          PathTerm *E = s_terms + warp * 64;
-          const unsigned m0 = __ballot_sync(0xffffffffu, in[0]), m1 = __ballot_sync(0xffffffffu, in[kStep - 1]);
-          const unsigned below = (1u << lane) - 1u;
-          const int n0 = __popc(m0), nt = n0 + __popc(m1);
-          if (in[0]) E[__popc(m0 & below)] = tt[0];
-          if (in[kStep - 1]) E[n0 + __popc(m1 & below)] = tt[kStep - 1];
+          // lanes: a cell's node pair is one 128-byte line a team, against a line
+          // a lane.
           __syncwarp();
-          for (int x = lane >> 2; x < nt; x += 8) {
-            const PathTerm P = E[x];
-            du += tricubic_team_part(tb.F, a.pa.t64, P.cell, P.u, lane & 3);
-          }
+          for (int x = lane >> 2; x < listed; x += 8) du += team_part(tb.F, a.pa.t64, E[x], lane & 3);
           __syncwarp();
         }
       }
@@ -459,9 +494,9 @@ cudaError_t launch_pair_path(const ReduceTarget &t, const double *path, const De
 #define PIMC_PAIR_PATH(KIND)                                                                                        \
   do {                                                                                                              \
     if (do_v)                                                                                                       \
-      pair_path_kernel<KIND, true><<<blocks, kThreads, 0, t.stream>>>(a, partials, t.counter, t.out);              \
+      pair_path_kernel<KIND, true><<<blocks, kThreadsOf<KIND>, 0, t.stream>>>(a, partials, t.counter, t.out);              \
     else                                                                                                            \
-      pair_path_kernel<KIND, false><<<blocks, kThreads, 0, t.stream>>>(a, partials, t.counter, t.out);             \
+      pair_path_kernel<KIND, false><<<blocks, kThreadsOf<KIND>, 0, t.stream>>>(a, partials, t.counter, t.out);             \
   } while (0)
   if (pa.kind == PA_DAVID)
     PIMC_PAIR_PATH(PA_DAVID);
