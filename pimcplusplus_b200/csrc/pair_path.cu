@@ -34,6 +34,12 @@ namespace pimc {
 namespace {
 
 constexpr int kMaxTile = 64;
+// With lists a block takes one i tile against up to kGroup j tiles: their pairs
+// gather in one list, so the walks fill the block although few of a tile's pairs
+// survive (the energy of N = 4096, M = 256, a range of 0.11 box sides: 560 us
+// with a list a tile pair, 513 in groups).
+constexpr int kGroup = 8;
+constexpr int kListMax = kMaxTile * kMaxTile + 1024;  // walked when past 1024: the next tile fits
 // Threads a block (tricubic, N = 512: 128 threads 625 us, 256 608; N = 37: 32.6, 34.3)
 template <int KIND>
 constexpr int kThreadsOf = KIND == PA_TRICUBIC ? 128 : 256;
@@ -44,7 +50,7 @@ struct PairPathArgs {
   DevPA pa;
   int slice1, skip, nlinks, level;
   int tile_log2, chunk;      // particles per tile (log2), links per chunk
-  long long ntp, items;      // tile pairs; tile pairs x chunks
+  long long ntp, items;      // tile pairs (with lists: tile x group pairs); those x chunks
   const float4 *bounds;      // [chunk][N] {centre, radius} or null (every pair is taken)
   double near2;              // (0.49 smallest box side)^2
 };
@@ -169,7 +175,7 @@ __global__ void __launch_bounds__(kThreadsOf<KIND>, KIND == PA_TRICUBIC ? 4 : 3)
   constexpr int kThreads = kThreadsOf<KIND>, kWarps = kThreads / 32;
   constexpr int kStep = KIND == PA_TRICUBIC ? 4 : 1;  // links between two gathers: their terms fill the teams' rounds
   __shared__ float4 s_bi[kMaxTile], s_bj[kMaxTile];
-  __shared__ unsigned short s_list[kMaxTile * kMaxTile];
+  __shared__ unsigned short s_list[kListMax];  // i << 9 | j in the group
   __shared__ int s_cnt[kWarps + 1];
   __shared__ PathTerm s_terms[KIND == PA_TRICUBIC ? kWarps * 32 * kStep : 1];
   PathTerm *const E = s_terms + (KIND == PA_TRICUBIC ? (threadIdx.x >> 5) * 32 * kStep : 0);
@@ -193,17 +199,34 @@ __global__ void __launch_bounds__(kThreadsOf<KIND>, KIND == PA_TRICUBIC ? 4 : 3)
   double du = 0.0, vs = 0.0;
   for (long long item = blockIdx.x; item < a.items; item += gridDim.x) {
     const int c = (int)(item / a.ntp);
-    int ti, tj;
-    tri_decode(item - c * a.ntp, ti, tj);
+    const bool lists = KIND == PA_DAVID && a.bounds;
+    int ti, tj, tj1;  // j tiles [tj, tj1)
+    if (lists) {
+      // groups of tile row ti: 0 .. ti / kGroup; rows [kGroup b, kGroup (b + 1)) have b + 1 each
+      const long long k = item - c * a.ntp;
+      int b, r;
+      tri_decode(k / kGroup, b, r);
+      const int rem = (int)(k - (long long)kGroup * b * (b + 1) / 2);
+      ti = kGroup * b + rem / (b + 1);
+      tj = kGroup * (rem % (b + 1));
+      tj1 = min(tj + kGroup, ti + 1);
+      if (ti << a.tile_log2 >= N) continue;  // the last row block's empty rows
+    } else {
+      tri_decode(item - c * a.ntp, ti, tj);
+      tj1 = tj + 1;
+    }
     const int i0 = ti << a.tile_log2, j0 = tj << a.tile_log2;
-    const int ni = min(T, N - i0), nj = min(T, N - j0);
+    const int ni = min(T, N - i0);
     const int lbeg = c * a.chunk, lend = min(a.nlinks, lbeg + a.chunk);
     int n = T << a.tile_log2;  // units' pairs: all (i, j) of the tiles, or the list
+    if (lists) n = 0;
+    for (int tc = tj; tc < tj1; tc++) {
+    const int jc = tc << a.tile_log2, nj = min(T, N - jc);
     if (KIND == PA_DAVID && a.bounds) {
       const float4 *bc = a.bounds + (size_t)c * N;
-      __syncthreads();  // the previous item's readers are done
-      if (tid < ni) s_bi[tid] = bc[i0 + tid];
-      if (tid >= kMaxTile && tid - kMaxTile < nj) s_bj[tid - kMaxTile] = bc[j0 + tid - kMaxTile];
+      __syncthreads();  // the previous readers are done
+      if (tc == tj && tid < ni) s_bi[tid] = bc[i0 + tid];
+      if (tid >= kMaxTile && tid - kMaxTile < nj) s_bj[tid - kMaxTile] = bc[jc + tid - kMaxTile];
       __syncthreads();
       // Warp w tests rows w, w + 8, ...: two lanes' worth of columns each; the
       // ballots stay in registers until the warps' counts give the places.
@@ -216,43 +239,43 @@ __global__ void __launch_bounds__(kThreadsOf<KIND>, KIND == PA_TRICUBIC ? 4 : 3)
 #pragma unroll
       for (int k = 0; k < kMaxTile / kWarps; k++) {
         const int i = warp + k * kWarps;
+        const float4 p = s_bi[i];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           const int j = lane + 32 * h;
-          bool take = i < ni && j < nj && (ti != tj || j < i);
-          if (take) {
-            const float4 p = s_bi[i], q = s_bj[j];
-            float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
-            dx -= rintf(dx * ix) * Lx;
-            dy -= rintf(dy * iy) * Ly;
-            dz -= rintf(dz * iz) * Lz;
-            const float lim = lim0 + p.w + q.w;
-            take = !(dx * dx + dy * dy + dz * dz > lim * lim);  // a NaN is taken: the sum reports it
-          }
+          const float4 q = s_bj[j];
+          float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+          dx -= round_even_magic(dx * ix) * Lx;
+          dy -= round_even_magic(dy * iy) * Ly;
+          dz -= round_even_magic(dz * iz) * Lz;
+          const float lim = lim0 + p.w + q.w;
+          const bool take = i < ni && j < (ti == tc ? min(i, nj) : nj) &&
+                            !(dx * dx + dy * dy + dz * dz > lim * lim);  // a NaN is taken: the sum reports it
           m[k][h] = __ballot_sync(0xffffffffu, take);
           cnt += __popc(m[k][h]);
         }
       }
       if (lane == 0) s_cnt[warp] = cnt;
       __syncthreads();
-      int at = 0;
-      n = 0;
+      int at = n, found = 0;
       for (int w = 0; w < kWarps; w++) {
-        if (w == warp) at = n;
-        n += s_cnt[w];
+        if (w == warp) at += found;
+        found += s_cnt[w];
       }
       const unsigned below = (1u << lane) - 1u;
+      const int jg = (tc - tj) << a.tile_log2;
 #pragma unroll
       for (int k = 0; k < kMaxTile / kWarps; k++)
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           if (m[k][h] >> lane & 1u)
-            s_list[at + __popc(m[k][h] & below)] = (unsigned short)((warp + k * kWarps) << 6 | (lane + 32 * h));
+            s_list[at + __popc(m[k][h] & below)] =
+                (unsigned short)((warp + k * kWarps) << 9 | (jg + lane + 32 * h));
           at += __popc(m[k][h]);
         }
-      __syncthreads();
+      n += found;
       if (tid == 0) {  // the pairs left out: the end value on every link
-        const int out_of_range = (ti == tj ? ni * (ni - 1) / 2 : ni * nj) - n;
+        const int out_of_range = (ti == tc ? ni * (ni - 1) / 2 : ni * nj) - found;
         du += (double)out_of_range * (double)(lend - lbeg) * tb.end.f;
         if (DO_V) {
           double w = (double)(lend - lbeg);
@@ -261,8 +284,10 @@ __global__ void __launch_bounds__(kThreadsOf<KIND>, KIND == PA_TRICUBIC ? 4 : 3)
           vs += (double)out_of_range * w * tb.end.v;
         }
       }
-      if (n == 0) continue;
+      if (n <= kListMax - kMaxTile * kMaxTile && tc + 1 < tj1) continue;  // room for the next tile
+      __syncthreads();
     }
+    if (n == 0) continue;
     // Few pairs: their walks are cut so that about two units come to a thread
     int nsub = 1;
     const int links = lend - lbeg;
@@ -277,8 +302,8 @@ __global__ void __launch_bounds__(kThreadsOf<KIND>, KIND == PA_TRICUBIC ? 4 : 3)
       bool live = u < units;
       if (KIND == PA_DAVID && a.bounds) {
         const int code = live ? s_list[e] : 0;
-        i = code >> 6;
-        j = code & 63;
+        i = code >> 9;
+        j = code & 511;
       } else {
         i = e >> a.tile_log2;
         j = e & (T - 1);
@@ -368,6 +393,8 @@ __global__ void __launch_bounds__(kThreadsOf<KIND>, KIND == PA_TRICUBIC ? 4 : 3)
         }
       }
       if (DO_V && live && l1 == a.nlinks) vs += 0.5 * va.v;
+    }
+    if (lists) n = 0;  // walked
     }
   }
   // this block's sums, then the last block adds every block's in block order
@@ -478,8 +505,8 @@ cudaError_t launch_pair_path(const ReduceTarget &t, const double *path, const De
   a.chunk = cull ? kBoundsChunk : 8;
   a.tile_log2 = 6;
   auto count = [&]() {
-    const long long nt = (sys.N + (1 << a.tile_log2) - 1) >> a.tile_log2;
-    a.ntp = nt * (nt + 1) / 2;
+    const long long nt = (sys.N + (1 << a.tile_log2) - 1) >> a.tile_log2, nb = (nt + kGroup - 1) / kGroup;
+    a.ntp = cull ? kGroup * nb * (nb + 1) / 2 : nt * (nt + 1) / 2;
     return a.ntp * ((nlinks + a.chunk - 1) / a.chunk);
   };
   while (count() < 4 * sm_count && a.tile_log2 > 4) a.tile_log2--;

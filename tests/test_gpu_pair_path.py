@@ -104,6 +104,13 @@ def test_range(end, last_zero):
         check(o, d, [(1, slices - 1, 0)])
 
 
+@pytest.mark.parametrize("n", [512, 513, 577, 1090])  # eight tiles, a ninth, a ragged row of groups, three rows
+@pytest.mark.parametrize("end", [2.0, 5.9])  # a group's pairs in one list, and in several
+def test_groups_of_tiles(n, end):
+    o, d = pair(n, 4, [20.0, 20.5, 21.0], end, step=0.3)
+    check(o, d, [(0, 3, 0)])
+
+
 @pytest.mark.parametrize("terms", [1, 2])
 @pytest.mark.parametrize("n,end", [(40, 5.0), (280, 3.2)])
 def test_offdiagonal_terms(n, end, terms):
