@@ -136,26 +136,30 @@ __device__ __forceinline__ double dist_one_slice(const double a[3], const double
 // 0.5) (ObservableCorrelation.cc:191-207, Grid.h:81-84); bins counted per block
 // in shared memory, then added to the 64-bit histogram.
 // A block takes (tile of particles) x (tile) x slice items: the tiles'
-// positions are boxed in FP64 and staged as FP32, and a pair's distance and
-// place on the grid are formed in FP32.  The place carries an error below
-// `err` bins (see launch_gofr); a pair nearer than that to a bin's edge, or
-// with a position FP32 cannot box, is binned from its FP64 distance, so the
-// counts are the FP64 evaluation's.  With FP64 distances and 64-bit index
-// arithmetic for every pair this took 138 us for N = 512, M = 128 and 100 bins
-// and was bound by the FP64 and integer work; it now takes 44 us (ncu), bound by
-// instruction issue (about 50 a pair).
+// positions are boxed in FP64 and staged as 32-bit fractions of the box, so a
+// difference wraps to the minimum image by itself; a pair's distance, in bins,
+// and its place on the grid are formed from it in FP32.  The place carries an
+// error below `err` bins (see launch_gofr); a pair nearer than that to a bin's
+// edge, and every pair of two tiles with a position that the fractions cannot
+// hold, is binned from its FP64 distance, so the counts are the FP64
+// evaluation's.  Bound by instruction issue (75 %, 42 instructions a pair).
+// N = 512, M = 128, 100 bins (ncu): 138 us with FP64 distances and 64-bit index
+// arithmetic for every pair, 44 with FP32 coordinates and the image by rounding,
+// 40 with the fractions, 34 with the open pairs noted and binned after the rows
+// instead of a branch at each.  Tiles of 128: 52, too few items to share out evenly.
 template <int JPL>  // j particles per lane: tiles of 32 JPL particles
 __global__ void __launch_bounds__(256, 4) gofr_kernel(const double *__restrict__ path, DevSystem sys, GofrGrid gg,
-                                                   long long items, float err, float past,
-                                                   unsigned long long *hist) {
+                                                      long long items, float half, unsigned long long *hist) {
   constexpr int T = 32 * JPL;
   extern __shared__ unsigned int s_hist[];
-  __shared__ float4 s_pos[2 * T];  // the i tile, then the j tile
-  const int N = sys.N, S1 = sys.S - 1, tid = threadIdx.x, lane = tid & 31;
+  __shared__ int4 s_pos[2 * T];  // the i tile, then the j tile
+  const int N = sys.N, S1 = sys.S - 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < gg.nbins; i += blockDim.x) s_hist[i] = 0u;
-  const float Lx = (float)sys.box[0], Ly = (float)sys.box[1], Lz = (float)sys.box[2];
-  const float ix = (float)sys.boxinv[0], iy = (float)sys.boxinv[1], iz = (float)sys.boxinv[2];
-  const float dinv = (float)gg.deltainv, t0 = (float)(gg.start * gg.deltainv);
+  // squares of the bins in a 2^32nd of each box side; the grid start and half a bin, in bins
+  const double ux = 0x1p-32 * sys.box[0] * gg.deltainv, uy = 0x1p-32 * sys.box[1] * gg.deltainv,
+               uz = 0x1p-32 * sys.box[2] * gg.deltainv;
+  const float sx = (float)(ux * ux), sy = (float)(uy * uy), sz = (float)(uz * uz);
+  const float t0 = (float)(gg.start * gg.deltainv + 0.5);
   // A block takes consecutive items, slice fastest, so it divides once.
   const long long beg = items * blockIdx.x / gridDim.x, end = items * (blockIdx.x + 1) / gridDim.x;
   int ti, tj, slice = (int)(beg % S1);
@@ -165,49 +169,52 @@ __global__ void __launch_bounds__(256, 4) gofr_kernel(const double *__restrict__
     const int ni = min(T, N - i0), nj = min(T, N - j0);
     const double *row = path + (size_t)slice * N * 3;
     __syncthreads();  // the previous item's readers are done
+    bool far = false;
     if (tid < 2 * T) {
       const int p = tid < T ? i0 + tid : j0 + tid - T;
       if (p < N) {
-        float v[3];
+        int v[3];
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-          const double x = row[(size_t)p * 3 + d], b = sys.box[d];
-          const double boxed = x - round_even_magic(x * sys.boxinv[d]) * b;
-          v[d] = fabs(x) <= 1e6 * b ? (float)boxed : __int_as_float(0x7fffffff);  // NaN: FP64 for its pairs
+          const double f = row[(size_t)p * 3 + d] * sys.boxinv[d];
+          far |= !(fabs(f) <= 1e6);
+          v[d] = (int)(unsigned)__double2ll_rn((f - round_even_magic(f)) * 0x1p32);  // both halves: -2^31
         }
-        s_pos[tid] = make_float4(v[0], v[1], v[2], 0.0f);
+        s_pos[tid] = make_int4(v[0], v[1], v[2], 0);
       }
     }
-    __syncthreads();
-    float4 q[JPL];
+    const float lim = __syncthreads_or(far) ? -1.0f : half;
+    int4 q[JPL];
 #pragma unroll
     for (int h = 0; h < JPL; h++) q[h] = s_pos[T + lane + 32 * h];
-#pragma unroll 2
-    for (int i = tid >> 5; i < ni; i += 8) {
-      const float4 p = s_pos[i];
-      const int jend = ti == tj ? i : nj;
+    unsigned edges = 0u;  // this lane's pairs that FP32 leaves open, binned below: no branch in the loop
+#pragma unroll
+    for (int r = 0; r < T / 8; r++) {
+      const int i = warp + 8 * r;
+      const int4 p = s_pos[i];
+      const int jend = i < ni ? (ti == tj ? i : nj) : 0;
 #pragma unroll
       for (int h = 0; h < JPL; h++) {
-        const int j = lane + 32 * h;
-        float dx = q[h].x - p.x, dy = q[h].y - p.y, dz = q[h].z - p.z;
-        dx -= round_even_magic(dx * ix) * Lx;
-        dy -= round_even_magic(dy * iy) * Ly;
-        dz -= round_even_magic(dz * iz) * Lz;
+        const float dx = (float)(int)((unsigned)q[h].x - (unsigned)p.x), dy = (float)(int)((unsigned)q[h].y - (unsigned)p.y),
+                    dz = (float)(int)((unsigned)q[h].z - (unsigned)p.z);
         float dist;
-        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(dist) : "f"(dx * dx + dy * dy + dz * dz));
-        const float t = dist * dinv - t0;
-        if (t > past || j >= jend) continue;
-        const float low = round_even_magic(t - 0.5f), e = t - low;
-        int bin = int_of_integral(low);
-        if (!(e > err && e < 1.0f - err)) {
-          double a[3], b[3];
-          load3(row + (size_t)(i0 + i) * 3, a);
-          load3(row + (size_t)(j0 + j) * 3, b);
-          const double d64 = dist_one_slice(a, b, sys);
-          bin = d64 < gg.end ? (int)rint(rsub(rmul(rsub(d64, gg.start), gg.deltainv), 0.5)) : -1;
-        }
-        if ((unsigned)bin < (unsigned)gg.nbins) atomicAdd(&s_hist[bin], 1u);
+        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(dist) : "f"(dx * dx * sx + dy * dy * sy + dz * dz * sz));
+        const float t = dist - t0, m = __fadd_rn(t, 12582912.0f);  // t's integer, as in round_even_magic
+        const unsigned bin = __float_as_uint(m) - 0x4B400000u;
+        const bool in = lane + 32 * h < jend, sure = fabsf(t - __fadd_rn(m, -12582912.0f)) < lim;
+        if (in && !sure) edges |= 1u << (r * JPL + h);
+        if (in && sure && bin < (unsigned)gg.nbins) atomicAdd(&s_hist[bin], 1u);
       }
+    }
+    while (edges) {
+      const int k = __ffs(edges) - 1, i = warp + 8 * (k / JPL), j = lane + 32 * (k % JPL);
+      edges &= edges - 1u;
+      double a[3], b[3];
+      load3(row + (size_t)(i0 + i) * 3, a);
+      load3(row + (size_t)(j0 + j) * 3, b);
+      const double d64 = dist_one_slice(a, b, sys);
+      const int bin = d64 < gg.end ? (int)rint(rsub(rmul(rsub(d64, gg.start), gg.deltainv), 0.5)) : -1;
+      if ((unsigned)bin < (unsigned)gg.nbins) atomicAdd(&s_hist[bin], 1u);
     }
     if (++slice == S1) {
       slice = 0;
@@ -371,20 +378,24 @@ cudaError_t launch_kin_dbeta(const ReduceTarget &t, const double *path, const De
   return cudaGetLastError();
 }
 
-// err, in bins, with u = 2^-24: a boxed coordinate rounds by L u / 2; the
-// difference of two by L u, its image by L u (the FP32 box side) + L u / 2: with
-// both coordinates 3.5 L u a dimension, sqrt(3) times that for the distance, and
-// the squares, their sum and the root (2^-22 of itself at most) add 6.5 u of a
-// distance up to 0.87 L; start deltainv rounds by u of itself and the place by 3 u
-// of itself, at most the bins to the box diagonal.  16 L u deltainv + 4 u (nbins + start deltainv)
-// holds them all.  The bound on |x| leaves the FP64 distance's own rounding
-// (1e6 L 2^-52) far below that.  From 1/2 on every pair takes the FP64 path, as
-// for boxes whose squares FP32 does not hold.
+// err, in bins, with u = 2^-24.  A coordinate's fraction: 2^-33 for the integer
+// and 1e6 2^-52 for boxing; the FP64 distance's own rounding at such a coordinate
+// is as large: below 2^-29 of the side for a difference, twice that where the two
+// choose different images at half a box, sqrt(3) times that for the distance:
+// 2^-27 L.  The conversion, the squares, the scales and the sum round by 7 u of
+// the square, the root by 4 u: 7.5 u of a distance, the start and the place by
+// 2 u of themselves, at most nbins + 1 bins beyond the start where it counts.
+// From 1/2 on every pair takes the FP64 path, as for boxes of less than 1e-6 or
+// more than 1e6 bins, which the FP32 squares and the rounding do not hold.
 cudaError_t launch_gofr(cudaStream_t st, const double *path, const DevSystem &sys, const GofrGrid &gg,
                         unsigned long long *hist, int sm_count) {
-  const double L = fmax(sys.box[0], fmax(sys.box[1], sys.box[2]));
-  double err = (16.0 * L * gg.deltainv + 4.0 * (gg.nbins + gg.start * gg.deltainv)) * 5.9604644775390625e-8;
-  if (!(L < 1e15 && L > 1e-15)) err = HUGE_VAL;
+  double err = 0.0;
+  for (double L : sys.box) {
+    const double bins = L * gg.deltainv;
+    err = fmax(err, bins > 1e-6 && bins < 1e6 ? bins * 0x1p-27 : HUGE_VAL);
+  }
+  err += 16.0 * (gg.nbins + 2 + fabs(gg.start * gg.deltainv)) * 0x1p-24;
+  const float half = fmax(0.5 - err, -1.0);  // a place nearer than this to its bin's centre is sure
   auto count = [&](int tile) {
     const long long nt = (sys.N + tile - 1) / tile;
     return nt * (nt + 1) / 2 * (sys.S - 1);
@@ -397,7 +408,7 @@ cudaError_t launch_gofr(cudaStream_t st, const double *path, const DevSystem &sy
   const cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              12288 * (int)sizeof(unsigned int));  // beside the static tiles
   if (e != cudaSuccess) return e;
-  kfn<<<blocks, 256, dyn, st>>>(path, sys, gg, items, (float)err, (float)(gg.nbins + 1 + err), hist);
+  kfn<<<blocks, 256, dyn, st>>>(path, sys, gg, items, half, hist);
   return cudaGetLastError();
 }
 

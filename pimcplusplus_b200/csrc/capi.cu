@@ -259,9 +259,13 @@ int pimc_create(const pimc_system_desc *d, pimc_context **out) {
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_partials, kPartialSlots * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_counter, sizeof(unsigned int));
   if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned int), ctx->stream);
-  if (e == cudaSuccess)  // one pinned page: the scalars, then the states of a sequential chain or of every window
-    e = cudaMallocHost(&ctx->h_out, 4 * sizeof(double) + kMaxWindows * sizeof(ChainState));
-  if (e == cudaSuccess) ctx->h_chain = reinterpret_cast<ChainState *>(ctx->h_out + 4);
+  if (e == cudaSuccess)  // one pinned block: the scalars, the states of a sequential chain or of every window, bins
+    e = cudaMallocHost(&ctx->h_out, 4 * sizeof(double) + kMaxWindows * sizeof(ChainState) +
+                                        kPinnedBins * sizeof(unsigned long long));
+  if (e == cudaSuccess) {
+    ctx->h_chain = reinterpret_cast<ChainState *>(ctx->h_out + 4);
+    ctx->h_bins = reinterpret_cast<unsigned long long *>(ctx->h_chain + kMaxWindows);
+  }
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_bounds, pair_path_bounds_bytes(s.N, s.S));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_chain, kMaxChainStates * sizeof(ChainState));
   if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_chain, 0, kMaxChainStates * sizeof(ChainState), ctx->stream);
@@ -295,7 +299,7 @@ int pimc_destroy(pimc_context *ctx) {
   cudaFree(ctx->d_dulong_k);
   cudaFree(ctx->d_yk);
   cudaFree(ctx->d_gofr);
-  if (ctx->h_gofr) cudaFreeHost(ctx->h_gofr);
+  if (ctx->h_gofr && ctx->h_gofr != ctx->h_bins) cudaFreeHost(ctx->h_gofr);
   cudaFree(ctx->d_kvec);
   cudaFree(ctx->d_nbr_cb);
   cudaFree(ctx->d_nbr_cnt);
@@ -1264,9 +1268,12 @@ int pimc_gofr_setup(pimc_context *ctx, double start, double end, int num_points)
   CK(cudaSetDevice(ctx->device));
   cudaFree(ctx->d_gofr);
   ctx->d_gofr = nullptr;
-  if (ctx->h_gofr) cudaFreeHost(ctx->h_gofr);
-  ctx->h_gofr = nullptr;
-  CK(cudaMallocHost(&ctx->h_gofr, (size_t)(num_points - 1) * sizeof(unsigned long long)));
+  if (ctx->h_gofr && ctx->h_gofr != ctx->h_bins) cudaFreeHost(ctx->h_gofr);
+  ctx->h_gofr = ctx->h_bins;
+  if (num_points - 1 > kPinnedBins) {  // a pinned allocation costs up to milliseconds: only for long histograms
+    ctx->h_gofr = nullptr;
+    CK(cudaMallocHost(&ctx->h_gofr, (size_t)(num_points - 1) * sizeof(unsigned long long)));
+  }
   CK(cudaMalloc(&ctx->d_gofr, (size_t)(num_points - 1) * sizeof(unsigned long long)));
   CK(cudaMemsetAsync(ctx->d_gofr, 0, (size_t)(num_points - 1) * sizeof(unsigned long long), ctx->stream));
   ctx->gofr_points = num_points;

@@ -138,6 +138,7 @@ struct DevSystem {
 };
 
 constexpr int kMaxWindows = 64;      // concurrent slice windows of one chain
+constexpr int kPinnedBins = 512;     // g(r) bins that fit the pinned block of the results
 constexpr uint32_t kStreamLocal = 0, kStreamCommon = 1, kStreamWorld = 2;
 // Local stream of window w, proposal slot p (slot 0 without proposals) is
 // kStreamWindow0 + p * kMaxWindows + w, in ChainState p * kMaxWindows + w
@@ -219,7 +220,8 @@ struct pimc_context {
   double *d_yk = nullptr;
   bool yk_ready = false;
   // pair correlation accumulator (PairCorrelationClass)
-  unsigned long long *d_gofr = nullptr, *h_gofr = nullptr;  // device bins; pinned copy
+  unsigned long long *d_gofr = nullptr, *h_gofr = nullptr;  // device bins; pinned copy: h_bins, or its own
+  unsigned long long *h_bins = nullptr;                     // behind h_chain: kPinnedBins
   int gofr_points = 0;
   double gofr_start = 0, gofr_end = 0, gofr_delta = 0, gofr_deltainv = 0;
   long long gofr_counts = 0;
