@@ -1509,6 +1509,15 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
         S.tot.c.reevals += S.mv.reevals;
       }
     };
+    // The stream table is refilled once less than half of it is ahead of the
+    // committed position (the next move's draws, if any, are committed).  All
+    // warps take the same turn, because the fill holds the group's barriers: each
+    // reads the position before a barrier that the sampler, which moves it on when
+    // no next move was speculated, has yet to pass.
+    auto refill_due = [&]() {
+      return (long long)(S.tab.tb + (uint64_t)S.tab.W) - (long long)s_rng.n < (long long)(tab_mem.W >> 1);
+    };
+    bool refill;
     if (!PROP) {
       if (acc_all && move_far) {
         // this move left its sphere: the lists no longer bound this job's
@@ -1527,7 +1536,8 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
       take_record();
       if (counter) count_move();
       if (have_next) cur ^= 1;
-      G.sync();  // every thread has read s_ctl / s_next before the next move rewrites them
+      refill = refill_due();
+      G.sync();  // every thread has read s_ctl / s_next / s_rng before the next move rewrites them
       if (meet) cluster_arrive(writer || a.use_lr);
       put_record(a.concurrent ? (long long)window * a.steps_per_block + m : (long long)m);
       if (++bstep == a.steps_per_block) bstep = 0;
@@ -1606,11 +1616,10 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
         pfirst = nf;
       }
       if (S.s_commit[1]) break;
+      refill = refill_due();  // behind the cluster barrier: a redo has set the position back
+      G.sync();
     }
-    // Refill the stream table once less than half of it is ahead of the
-    // committed position (the next move's draws, if any, are committed).
-    if ((long long)(S.tab.tb + (uint64_t)S.tab.W) - (long long)s_rng.n < (long long)(tab_mem.W >> 1))
-      rng_tab_fill(S.tab, tab_mem.W, seed, stream, s_rng.n, tid, G.size, gsync);
+    if (refill) rng_tab_fill(S.tab, tab_mem.W, seed, stream, s_rng.n, tid, G.size, gsync);
   }
   if (lead) {
     cs->nlocal = s_rng.n;
