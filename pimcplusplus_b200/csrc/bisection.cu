@@ -1356,7 +1356,11 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
           // commit the stream position the outcome selects
           const bool ends = !toAccept || level == 0 || status != 0;
           if (lane == 0) {
-            S.s_need[0] = 0;
+            // Not behind a re-evaluation: the warps that take no part in it (the
+            // speculator, and the sampler where it sums no kinetic links) may still
+            // be reading the flag that sends them through its closing barrier.  The
+            // next stage's first decision, which waits for every warp, rewrites it.
+            if (!exact) S.s_need[0] = 0;
             s_ctl[2] = toAccept ? 1 : 0;
             s_ctl[3] = status;
             int nv = 0;

@@ -9,6 +9,7 @@ import pimcplusplus_b200 as P
 from pimcplusplus_b200 import workloads as W
 
 from helpers import lj_case
+from test_gpu_batch import make_chains, oracle_run
 from test_gpu_parity import compare_traces, run_trace_pair
 from test_gpu_proposals import _c5_pair, _compare
 
@@ -54,3 +55,53 @@ def test_stream_table_refills_proposals(tmp_path, warps):
     assert stats["moves"] == len(live) and stats["status"] == 0 and stats["redone"] > 0
     assert np.max(np.abs(d.get_path(P.OLDMODE) - o.get_path(0))) < 1e-9
     d.close()
+
+
+@pytest.mark.parametrize("cluster", [1, 3])
+@pytest.mark.parametrize("warps", WARPS)
+def test_every_stage_reevaluated(tmp_path, warps, cluster):
+    """The relative guard re-evaluates stage after stage in FP64; warps without a part in that pass it by."""
+    o, d = system(tmp_path, 40)
+    ref, got, stats = run_trace_pair(o, d, 3, 4, 60, 11, precision=P.MIXED, guard=P.GUARD_RELATIVE,
+                                     cluster_ctas=cluster, threads_per_cta=32 * warps)
+    compare_traces(ref, got, stats)
+    assert stats["reevaluated"] > 0.5 * stats["stages_attempted"]
+    assert np.max(np.abs(d.get_path(P.OLDMODE) - o.get_path(0))) < 1e-9
+    d.close()
+
+
+@pytest.mark.parametrize("warps", [2, 4, 6, 8])
+def test_every_stage_reevaluated_proposals(tmp_path, warps):
+    o, d, L = _c5_pair(tmp_path, 64, 128, 17)
+    o.bisection_config(L, 3)
+    o.rng_seed(19)
+    bb = P.BisectionBlock(d, L, 3, schedule=P.PROPOSALS, cluster_ctas=4, threads_per_cta=32 * warps,
+                          precision=P.MIXED, guard=P.GUARD_RELATIVE)
+    bb.seed(19)
+    got, stats = bb.MakeMoves(4)
+    ref = list(o.run_proposals(4, 4))
+    live = [(r, g) for r, g in zip(ref, got) if r.slice1 >= 0]
+    assert len(ref) == len(got) and stats["moves"] == len(live) and stats["status"] == 0
+    for i, (r, g) in enumerate(live):
+        assert (r.slice1, r.ptcl, r.accepted, r.stages_passed) == (
+            int(g["slice1"]), int(g["ptcl"]), int(g["accepted"]), int(g["stages_passed"])), i
+    assert stats["reevaluated"] > 0
+    assert np.max(np.abs(d.get_path(P.OLDMODE) - o.get_path(0))) < 1e-9
+    d.close()
+
+
+@pytest.mark.parametrize("threads,max_split", [(64, 0), (128, 0), (160, 0), (192, 0), (256, 2), (512, 1), (512, 2)])
+def test_every_stage_reevaluated_batch(threads, max_split):
+    chains = make_chains()
+    b = P.BatchChains(chains, precision=P.MIXED, threads_per_cta=threads, ctas=5, max_split=max_split)
+    b.set_guard(P.GUARD_RELATIVE)
+    trace, stats = b.run(20, trace=True)
+    assert stats["status"] == 0 and stats["reevaluated"] > 0.5 * stats["stages_attempted"]
+    for i, c in enumerate(chains):
+        ref, ref_path, _ = oracle_run(c, 20)
+        for k, r in enumerate(ref):
+            g = trace[i][k]
+            assert (r.slice1, r.ptcl, r.accepted, r.stages_passed) == (
+                int(g["slice1"]), int(g["ptcl"]), int(g["accepted"]), int(g["stages_passed"])), (i, k)
+        assert np.max(np.abs(b.path(i) - ref_path)) < 1e-9, i
+    b.close()
