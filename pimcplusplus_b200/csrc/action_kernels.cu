@@ -9,6 +9,7 @@
 
 #include "action_kernels.cuh"
 #include "device_math.cuh"
+#include "gofr_shape.h"
 
 namespace pimc {
 
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(256, 4) gofr_kernel(const double *__restrict__
   const float sx = (float)(ux * ux), sy = (float)(uy * uy), sz = (float)(uz * uz);
   const float t0 = (float)(gg.start * gg.deltainv + 0.5);
   // A block takes consecutive items, slice fastest, so it divides once.
-  const long long beg = items * blockIdx.x / gridDim.x, end = items * (blockIdx.x + 1) / gridDim.x;
+  const long long beg = gofr_first(items, gridDim.x, blockIdx.x), end = gofr_first(items, gridDim.x, blockIdx.x + 1ll);
   int ti, tj, slice = (int)(beg % S1);
   tri_decode(beg / S1, ti, tj);
   for (long long item = beg; item < end; item++) {
@@ -396,19 +397,13 @@ cudaError_t launch_gofr(cudaStream_t st, const double *path, const DevSystem &sy
   }
   err += 16.0 * (gg.nbins + 2 + fabs(gg.start * gg.deltainv)) * 0x1p-24;
   const float half = fmax(0.5 - err, -1.0);  // a place nearer than this to its bin's centre is sure
-  auto count = [&](int tile) {
-    const long long nt = (sys.N + tile - 1) / tile;
-    return nt * (nt + 1) / 2 * (sys.S - 1);
-  };
-  const bool wide = count(64) >= 4 * sm_count;  // tiles of 64 unless they leave the SMs short of blocks
-  const long long items = count(wide ? 64 : 32);
-  const int blocks = (int)std::min(items, (long long)4 * sm_count);  // all resident
+  const GofrShape shape = gofr_shape(sys.N, sys.S - 1, sm_count);
   const size_t dyn = (size_t)gg.nbins * sizeof(unsigned int);
-  auto kfn = wide ? gofr_kernel<2> : gofr_kernel<1>;
+  auto kfn = shape.tile == 64 ? gofr_kernel<2> : gofr_kernel<1>;
   const cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              12288 * (int)sizeof(unsigned int));  // beside the static tiles
   if (e != cudaSuccess) return e;
-  kfn<<<blocks, 256, dyn, st>>>(path, sys, gg, items, half, hist);
+  kfn<<<shape.blocks, 256, dyn, st>>>(path, sys, gg, shape.items, half, hist);
   return cudaGetLastError();
 }
 
