@@ -98,7 +98,8 @@ template <int KIND, bool DO_V>
 __device__ __forceinline__ SliceVal slice_value(const DevPA &pa, const Tables<KIND> &t, double r) {
   if (KIND == PA_DAVID) {
     const DDavid<double> &d = pa.d64;
-    if (r >= d.grid.end) return t.end;
+    // a length that overflowed is not "beyond the table": the spline makes it NaN, which is reported
+    if (r >= d.grid.end && __double2hiint(r) != 0x7ff00000) return t.end;
     return david_slice<DO_V>(d, t.est, t.est0, r < d.grid.start ? d.grid.start : r);
   }
   SliceVal s;

@@ -155,3 +155,18 @@ def test_non_finite_positions_are_reported(n, end):
                 call()
             assert e.value.status == 3
         d.close()
+
+
+@pytest.mark.parametrize("n,end", [(20, 4.0), (300, 2.9)])
+@pytest.mark.parametrize("rows", [[17], [16, 17, 18], list(range(40))])
+def test_overflowing_distances_are_reported(n, end, rows):
+    """Positions whose squared distance overflows: no pair of theirs has a length, so no sum of theirs is a number."""
+    o, d = pair(n, 40, [10.0] * 3, end, last_zero=False)
+    path = d.get_path()
+    path[rows, n - 3, 1] = 1e200
+    d.set_path(path)
+    for call in (d.energy, lambda: d.d_dbeta(P.ACTION_SHORTRANGE, 0, 39, 0)):
+        with pytest.raises(P.PimcError) as e:
+            call()
+        assert e.value.status == 3
+    d.close()
