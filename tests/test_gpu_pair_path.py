@@ -170,3 +170,17 @@ def test_overflowing_distances_are_reported(n, end, rows):
             call()
         assert e.value.status == 3
     d.close()
+
+
+@pytest.mark.parametrize("n", [5, 32, 70])
+def test_coulomb_long_steps_with_the_potential(n):
+    """Links longer than half the box in the walk that carries V: heavier zero-point motion than in
+    test_tricubic_and_coulomb keeps the kinetic estimator finite there, so d_dBeta and V are compared."""
+    box = np.array([12.0, 12.0, 12.0])
+    path = random_walk_path(n, 11, box, 4.0, n, far=0.1)
+    o = Oracle(n, box, W.HE4_LAMBDA, O.PairAction.classical_coulomb(TAU, LEVELS, 2.0), path)
+    assert math.isfinite(o.energy()["kinetic"])
+    d = P.PathData(n, 11, box, TAU, W.HE4_LAMBDA, 0)
+    d.pa_coulomb(2.0, LEVELS)
+    d.set_path(path)
+    check(o, d, [(0, 10, 0), (1, 9, 2)])
