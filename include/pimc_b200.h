@@ -254,8 +254,10 @@ typedef struct pimc_bisection_desc {
   int use_longrange;                /* LongRange pushed at the lowest level */
   int precision;                    /* PIMC_FP64 or PIMC_MIXED */
   int shadow;                       /* also evaluate the other precision, for dS error */
-  int cluster_ctas;                 /* CTAs cooperating on one chain (1..16), 0 = auto (by N, levels and schedule);
-                                       PROPOSALS: proposal slots per window (2..16), one CTA each */
+  int cluster_ctas;                 /* CTAs cooperating on one chain (1..16), 0 = auto (by N, levels, k-vectors and
+                                       schedule, for one context that has the GPU; a program that runs many
+                                       contexts at once sets it smaller for chains of some 500 particles up, or
+                                       uses pimc_batch_*); PROPOSALS: proposal slots per window (2..16), one CTA each */
   int threads_per_cta;              /* 0 = auto */
   int schedule;                     /* PIMC_SCHEDULE_SEQUENTIAL, _WINDOWS or _PROPOSALS */
   /* Neighbour lists for the short-range sum (the role of ShortRangeOnClass's

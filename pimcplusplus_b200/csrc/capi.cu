@@ -700,6 +700,16 @@ static int window_slots(const pimc_context *ctx, int num_levels) {
 // With concurrent windows the clusters are halved until every window's fits on
 // the GPU at once: a second wave costs more (N = 64, L = 1, 32 windows: 4 x 256
 // 6.2, 8 x 512 17.1).  Proposals keep 8 slots.
+// The rule is for one context that has the GPU.  Several contexts' chains at once,
+// a host thread each, thousands of moves a second in all, this rule against the
+// fixed shape of before (1 x 256 below 256 particles, else 8 x 256), L = 3:
+//   8 hardware queues (the driver's default), 8 / 16 / 64 contexts:
+//     N = 64: 1166 / 1147 / 1071 against 714 / 689 / 638;  N = 512: 347 / 459 / 545 against 428 / 427 / 420
+//   32 queues (CUDA_DEVICE_MAX_CONNECTIONS), 16 / 32 / 64 contexts:
+//     N = 64: 2083 / 1802 / 1710 against 1157 / 1119 / 934;  N = 128: 1906 / 966 / 1395 against 902 / 926 / 863
+//     N = 512: 459 / 539 / 519 against 782 / 731 / 710
+// so only the 16-CTA shape costs such a program something: seven of its clusters
+// fit on the GPU.  Set-up: 14 us for the queries.
 static int auto_launch(pimc_context *ctx) {
   pimc_bisection_desc &b = ctx->bis;
   const bool prop = b.schedule == PIMC_SCHEDULE_PROPOSALS;
