@@ -12,14 +12,15 @@
 // in every dimension, which one comparison of s^2 establishes; otherwise the
 // walk forms it as the reference does.
 // Blocks take (tile of particles) x (tile of particles) x (chunk of links).
-// For a 1-D table that ends well inside the box, a block first lists the
-// pairs of its tiles whose bounding spheres over the chunk come within the
-// table's range; all others contribute the table's end value on every link.
+// For a 1-D table that ends well inside the box, and enough pairs (see
+// launch_pair_path), a block first lists the pairs of its tiles whose bounding
+// spheres over the chunk come within the table's range; all others contribute
+// the table's end value on every link.
 // Sums are taken in a fixed order, so results are bitwise reproducible.
 //
 // Measured as pimc_energy, against one thread per (pair, link) that decoded its
 // indices with 64-bit divisions and evaluated both ends of every link, and a
-// second such pass for V: N = 4096, M = 256, range 0.11 of the box 73.7 -> 0.57
+// second such pass for V: N = 4096, M = 256, range 0.11 of the box 73.7 -> 0.52
 // ms; N = 512, M = 128, tricubic 1042 -> 625 us; N = 128, M = 64, Coulomb
 // (both passes) 34 -> 22 us.  FP64 operations and their latencies bound it.
 #include <cuda_runtime.h>
@@ -40,7 +41,10 @@ constexpr int kMaxTile = 64;
 // with a list a tile pair, 513 in groups).
 constexpr int kGroup = 8;
 constexpr int kListMax = kMaxTile * kMaxTile + 1024;  // walked when past 1024: the next tile fits
-// Threads a block (tricubic, N = 512: 128 threads 625 us, 256 608; N = 37: 32.6, 34.3)
+// Threads a block.  Tricubic, 128 against 256 threads (pimc_energy, us): M = 128, N = 16
+// 30.5 / 28, 37 36.5 / 38, 64 46.6 / 46.2, 128 75.7 / 77, 192 140 / 134, 256 196 / 202, 384 440 / 399,
+// 512 660 / 638; M = 32, N = 64 32.8 / 35, 256 75.9 / 76, 512 191 / 193: neither is the better one
+// throughout, and no size tells them apart before 384.
 template <int KIND>
 constexpr int kThreadsOf = KIND == PA_TRICUBIC ? 128 : 256;
 
@@ -498,10 +502,23 @@ cudaError_t launch_pair_path(const ReduceTarget &t, const double *path, const De
   a.level = level;
   const double side = std::min(sys.box[0], std::min(sys.box[1], sys.box[2]));
   a.near2 = 0.49 * side * 0.49 * side;
-  // Bounding spheres pay when the range's sphere is a small part of the box:
-  // at 0.3 box sides it holds 11 % of the pairs (with the paths' own extent
-  // about a quarter).
-  const bool cull = pa.kind == PA_DAVID && sys.N >= 256 && pa.d64.grid.end <= 0.3 * side;
+  // Lists take long chunks and few items, so they cost a latency of their own and
+  // pay from a number of (pair, link)s on, the sooner the shorter the range: the
+  // times cross at about 5e7 range / side.  pimc_energy with / without, us, at 0.1,
+  // 0.2 and 0.3 sides:
+  //   N = 256, M = 16 (5e5):    68 / 40    95 / 42   123 / 40
+  //   N = 400, M = 64 (5e6):    87 / 84   130 / 100  190 / 108
+  //   N = 512, M = 64 (8e6):    93 / 109  147 / 127  200 / 136
+  //   N = 2048, M = 4 (8e6):    94 / 122  110 / 126  134 / 134
+  //   N = 512, M = 128 (17e6):  91 / 174  138 / 203  200 / 222
+  //   N = 4096, M = 2 (17e6):  104 / 225  135 / 244  187 / 261
+  //   N = 800, M = 64 (20e6):  104 / 235  164 / 278  250 / 309
+  //   N = 1200, M = 128 (92e6): 173 / 706  280 / 801  438 / 890
+  // (Beyond 0.3 sides they would gain 10-30 % from 3e7 on.  Below 256 particles, at
+  // 0.15 / 0.3 sides: N = 192, M = 256 74 / 128 with, 93 / 107 without; N = 128
+  // 75 / 133 and 60 / 64.)
+  const double end = pa.d64.grid.end, pair_links = 0.5 * sys.N * (sys.N - 1.0) * nlinks;
+  const bool cull = pa.kind == PA_DAVID && sys.N >= 256 && end <= 0.3 * side && pair_links * side >= 5e7 * end;
   a.bounds = cull ? bounds : nullptr;
   a.chunk = cull ? kBoundsChunk : 8;
   a.tile_log2 = 6;

@@ -184,3 +184,74 @@ def test_coulomb_long_steps_with_the_potential(n):
     d.pa_coulomb(2.0, LEVELS)
     d.set_path(path)
     check(o, d, [(0, 10, 0), (1, 9, 2)])
+
+
+class EndApart(Oracle):
+    """The oracle on tables less their end value, which every pair of every link adds and is multiplied out here: a
+    spline through y - c is the spline through y, less c.  Its running sum over a link's 1e5 like end values is off by
+    more than the bound."""
+
+    def __init__(self, n, box, end, npts, path):
+        start, end, u, du = david_tables(end, npts, 2, n, last_zero=False)
+        self.v, self.du = u[0, -1, 0], u[0, -1, 0] + du[0, -1, 1]
+        super().__init__(n, box, W.HE4_LAMBDA, O.PairAction.david_arrays(start, end, u - u[:, -1:], du - du[:, -1:], 0, 0),
+                         path)
+
+    def energy(self):
+        e, m, pairs = super().energy(), len(self.path) - 1, self.n * (self.n - 1) // 2
+        e["du_short"] += m * pairs * self.du
+        e["v_short"] += m * pairs * self.v
+        e["total"] = (e["kinetic"] + e["du_short"]) / m
+        return e
+
+    def shortrange_dbeta(self, s1, s2, level):
+        return super().shortrange_dbeta(s1, s2, level) + (s2 - s1 >> level) * (self.n * (self.n - 1) // 2) * self.du
+
+
+# Lists are taken from 5e7 range / side (pair, link)s on.  The cases above that were short of that go the general way
+# now; these reach the lists again, with the same edges: tiles, groups of tiles, chunks of links, ragged ends.
+@pytest.mark.parametrize("n,slices,end", [
+    (512, 39, 2.0), (512, 40, 2.0),  # 4.97e6 and 5.10e6 at 0.1 sides: either side of the line
+    (513, 41, 2.0), (577, 33, 2.0), (1090, 10, 2.0),  # a ninth tile, a ragged row of groups, three rows
+    (1090, 27, 5.9), (300, 331, 5.9),  # groups whose pairs fill several lists; eleven chunks of links, the last of ten
+    (256, 470, 5.9)])
+@pytest.mark.parametrize("last_zero", [True, False])
+def test_lists(n, slices, end, last_zero):
+    box = np.array([20.0, 20.5, 21.0])
+    o, d = pair(n, slices, box, end, step=0.3, last_zero=last_zero)
+    if not last_zero:
+        o = EndApart(n, box, end, 120, o.path)
+    check(o, d, [(0, slices - 1, 0), (1, slices - 1, 0)])
+
+
+@pytest.mark.parametrize("end", [2.0, 5.9])  # above the line at 0.1 sides, below it at 0.295
+def test_lists_one_link(end):
+    """Fifty rows of tiles.  With a table that ends at zero: the oracle's running sum over 5e6 like terms is off by
+    more than the bound."""
+    o, d = pair(3170, 2, [20.0, 20.5, 21.0], end, step=0.3)
+    check(o, d, [(0, 1, 0)])
+
+
+@pytest.mark.parametrize("terms", [1, 2])
+def test_lists_offdiagonal_terms(terms):
+    o, d = pair(280, 400, [11.0, 11.5, 12.0], 3.2, cols=7, terms=terms, tau_pos=1)
+    check(o, d, [(0, 399, 0)])
+
+
+def test_lists_long_steps():
+    o, d = pair(260, 450, [10.0] * 3, 2.9, step=4.0, far=0.3)
+    check(o, d, [(0, 448, 0)])
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, 1e200])
+@pytest.mark.parametrize("rows", [[170], [16, 17, 18], list(range(330))])
+def test_lists_report_non_finite_pairs(bad, rows):
+    o, d = pair(300, 330, [10.0] * 3, 2.9, last_zero=False)
+    path = d.get_path()
+    path[rows, 297, 1] = bad
+    d.set_path(path)
+    for call in (d.energy, lambda: d.d_dbeta(P.ACTION_SHORTRANGE, 0, 329, 0)):
+        with pytest.raises(P.PimcError) as e:
+            call()
+        assert e.value.status == 3
+    d.close()
