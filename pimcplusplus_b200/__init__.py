@@ -232,11 +232,12 @@ def _iptr(a):
 
 def _int_list(values):
     """(C int array, length) of a particle list.  A short list or tuple of plain
-    ints goes straight into a ctypes array: numpy and ndarray.ctypes cost several
-    us, a third of an action call; everything else takes numpy's conversion."""
+    ints goes straight into a ctypes array, each checked on the way: 0.7 us for one
+    and 1.8 for eight, where numpy and ndarray.ctypes take 2.6-2.9 (equal at
+    sixteen, 9.9 against 4.4 at sixty-four).  Everything else takes numpy's way."""
     if type(values) in (list, tuple):
         n = len(values)
-        if n <= 64 and all(type(v) is int and -0x80000000 <= v <= 0x7fffffff for v in values):
+        if n <= 8 and all(type(v) is int and -0x80000000 <= v <= 0x7fffffff for v in values):
             return (_i * n)(*values), n
     a = np.ascontiguousarray(values, dtype=np.int32)
     return _iptr(a), len(a)

@@ -62,3 +62,19 @@ def test_product_dm_reader_errors(tmp_path):
     p = write_testcoul_dm(str(tmp_path / "tc.dm"))
     with pytest.raises(P.PimcError):  # tau not on the file's tau grid
         P.read_dm(p, 0.3)
+
+
+@pytest.mark.parametrize("values", [[], [1], (2, 3), [2 ** 31 - 1, -2 ** 31], list(range(8)), list(range(9)),
+                                    list(range(64)), np.arange(3), np.arange(20, dtype=np.int64), [1.0, 2.0], [True],
+                                    [np.int64(3)], range(4), range(12)])
+def test_particle_lists_as_numpy_converts_them(values):
+    a, n = P._int_list(values)
+    assert [a[i] for i in range(n)] == list(np.ascontiguousarray(values, dtype=np.int32))
+
+
+@pytest.mark.parametrize("values", [[2 ** 31], [0] * 9 + [2 ** 31], [None], ["x"]])
+def test_particle_lists_that_numpy_refuses(values):
+    with pytest.raises(Exception) as e:
+        np.ascontiguousarray(values, dtype=np.int32)
+    with pytest.raises(e.type):
+        P._int_list(values)
