@@ -226,180 +226,180 @@ __global__ void __launch_bounds__(kThreadsOf<KIND>, KIND == PA_TRICUBIC ? 4 : 3)
     int n = T << a.tile_log2;  // units' pairs: all (i, j) of the tiles, or the list
     if (lists) n = 0;
     for (int tc = tj; tc < tj1; tc++) {
-    const int jc = tc << a.tile_log2, nj = min(T, N - jc);
-    if (KIND == PA_DAVID && a.bounds) {
-      const float4 *bc = a.bounds + (size_t)c * N;
-      __syncthreads();  // the previous readers are done
-      if (tc == tj && tid < ni) s_bi[tid] = bc[i0 + tid];
-      if (tid >= kMaxTile && tid - kMaxTile < nj) s_bj[tid - kMaxTile] = bc[jc + tid - kMaxTile];
-      __syncthreads();
-      // Warp w tests rows w, w + 8, ...: two lanes' worth of columns each; the
-      // ballots stay in registers until the warps' counts give the places.
-      const float Lx = (float)sys.box[0], Ly = (float)sys.box[1], Lz = (float)sys.box[2];
-      const float ix = (float)sys.boxinv[0], iy = (float)sys.boxinv[1], iz = (float)sys.boxinv[2];
-      // FP32 slack: centres, box sides and the image arithmetic round at 2^-24 of a box side each
-      const float lim0 = (float)a.pa.d64.grid.end * 1.000001f + 4e-6f * fmaxf(Lx, fmaxf(Ly, Lz));
-      unsigned m[kMaxTile / kWarps][2];
-      int cnt = 0;
-#pragma unroll
-      for (int k = 0; k < kMaxTile / kWarps; k++) {
-        const int i = warp + k * kWarps;
-        const float4 p = s_bi[i];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int j = lane + 32 * h;
-          const float4 q = s_bj[j];
-          float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
-          dx -= round_even_magic(dx * ix) * Lx;
-          dy -= round_even_magic(dy * iy) * Ly;
-          dz -= round_even_magic(dz * iz) * Lz;
-          const float lim = lim0 + p.w + q.w;
-          const bool take = i < ni && j < (ti == tc ? min(i, nj) : nj) &&
-                            !(dx * dx + dy * dy + dz * dz > lim * lim);  // a NaN is taken: the sum reports it
-          m[k][h] = __ballot_sync(0xffffffffu, take);
-          cnt += __popc(m[k][h]);
-        }
-      }
-      if (lane == 0) s_cnt[warp] = cnt;
-      __syncthreads();
-      int at = n, found = 0;
-      for (int w = 0; w < kWarps; w++) {
-        if (w == warp) at += found;
-        found += s_cnt[w];
-      }
-      const unsigned below = (1u << lane) - 1u;
-      const int jg = (tc - tj) << a.tile_log2;
-#pragma unroll
-      for (int k = 0; k < kMaxTile / kWarps; k++)
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          if (m[k][h] >> lane & 1u)
-            s_list[at + __popc(m[k][h] & below)] =
-                (unsigned short)((warp + k * kWarps) << 9 | (jg + lane + 32 * h));
-          at += __popc(m[k][h]);
-        }
-      n += found;
-      if (tid == 0) {  // the pairs left out: the end value on every link
-        const int out_of_range = (ti == tc ? ni * (ni - 1) / 2 : ni * nj) - found;
-        du += (double)out_of_range * (double)(lend - lbeg) * tb.end.f;
-        if (DO_V) {
-          double w = (double)(lend - lbeg);
-          if (lbeg == 0) w -= 0.5;
-          if (lend == a.nlinks) w += 0.5;
-          vs += (double)out_of_range * w * tb.end.v;
-        }
-      }
-      if (n <= kListMax - kMaxTile * kMaxTile && tc + 1 < tj1) continue;  // room for the next tile
-      __syncthreads();
-    }
-    if (n == 0) continue;
-    // Few pairs: their walks are cut so that about two units come to a thread
-    int nsub = 1;
-    const int links = lend - lbeg;
-    if (KIND == PA_DAVID && a.bounds)
-      while (n * nsub < 2 * kThreads && 4 * nsub < links) nsub *= 2;
-    const int len = (links + nsub - 1) / nsub;
-    const int units = n * nsub;
-    for (int u0 = 0; u0 < units; u0 += kThreads) {
-      const int u = u0 + tid;
-      const int sub = u / n, e = u - sub * n;
-      int i, j;
-      bool live = u < units;
+      const int jc = tc << a.tile_log2, nj = min(T, N - jc);
       if (KIND == PA_DAVID && a.bounds) {
-        const int code = live ? s_list[e] : 0;
-        i = code >> 9;
-        j = code & 511;
-      } else {
-        i = e >> a.tile_log2;
-        j = e & (T - 1);
-        live = live && i < ni && j < nj && (ti != tj || j < i);
+        const float4 *bc = a.bounds + (size_t)c * N;
+        __syncthreads();  // the previous readers are done
+        if (tc == tj && tid < ni) s_bi[tid] = bc[i0 + tid];
+        if (tid >= kMaxTile && tid - kMaxTile < nj) s_bj[tid - kMaxTile] = bc[jc + tid - kMaxTile];
+        __syncthreads();
+        // Warp w tests rows w, w + 8, ...: two lanes' worth of columns each; the
+        // ballots stay in registers until the warps' counts give the places.
+        const float Lx = (float)sys.box[0], Ly = (float)sys.box[1], Lz = (float)sys.box[2];
+        const float ix = (float)sys.boxinv[0], iy = (float)sys.boxinv[1], iz = (float)sys.boxinv[2];
+        // FP32 slack: centres, box sides and the image arithmetic round at 2^-24 of a box side each
+        const float lim0 = (float)a.pa.d64.grid.end * 1.000001f + 4e-6f * fmaxf(Lx, fmaxf(Ly, Lz));
+        unsigned m[kMaxTile / kWarps][2];
+        int cnt = 0;
+#pragma unroll
+        for (int k = 0; k < kMaxTile / kWarps; k++) {
+          const int i = warp + k * kWarps;
+          const float4 p = s_bi[i];
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int j = lane + 32 * h;
+            const float4 q = s_bj[j];
+            float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+            dx -= round_even_magic(dx * ix) * Lx;
+            dy -= round_even_magic(dy * iy) * Ly;
+            dz -= round_even_magic(dz * iz) * Lz;
+            const float lim = lim0 + p.w + q.w;
+            const bool take = i < ni && j < (ti == tc ? min(i, nj) : nj) &&
+                              !(dx * dx + dy * dy + dz * dz > lim * lim);  // a NaN is taken: the sum reports it
+            m[k][h] = __ballot_sync(0xffffffffu, take);
+            cnt += __popc(m[k][h]);
+          }
+        }
+        if (lane == 0) s_cnt[warp] = cnt;
+        __syncthreads();
+        int at = n, found = 0;
+        for (int w = 0; w < kWarps; w++) {
+          if (w == warp) at += found;
+          found += s_cnt[w];
+        }
+        const unsigned below = (1u << lane) - 1u;
+        const int jg = (tc - tj) << a.tile_log2;
+#pragma unroll
+        for (int k = 0; k < kMaxTile / kWarps; k++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            if (m[k][h] >> lane & 1u)
+              s_list[at + __popc(m[k][h] & below)] =
+                  (unsigned short)((warp + k * kWarps) << 9 | (jg + lane + 32 * h));
+            at += __popc(m[k][h]);
+          }
+        n += found;
+        if (tid == 0) {  // the pairs left out: the end value on every link
+          const int out_of_range = (ti == tc ? ni * (ni - 1) / 2 : ni * nj) - found;
+          du += (double)out_of_range * (double)(lend - lbeg) * tb.end.f;
+          if (DO_V) {
+            double w = (double)(lend - lbeg);
+            if (lbeg == 0) w -= 0.5;
+            if (lend == a.nlinks) w += 0.5;
+            vs += (double)out_of_range * w * tb.end.v;
+          }
+        }
+        if (n <= kListMax - kMaxTile * kMaxTile && tc + 1 < tj1) continue;  // room for the next tile
+        __syncthreads();
       }
-      const int l0 = lbeg + sub * len, l1 = min(lend, l0 + len);
-      live = live && l0 < l1;
-      if (KIND != PA_TRICUBIC && !live) continue;  // the tricubic teams need whole warps
-      const size_t row = (size_t)a.skip * N * 3;
-      const double *pi = a.path + ((size_t)(a.slice1 + (live ? l0 : lbeg) * a.skip) * N + i0 + (live ? i : 0)) * 3;
-      const double *pj = a.path + ((size_t)(a.slice1 + (live ? l0 : lbeg) * a.skip) * N + j0 + (live ? j : 0)) * 3;
-      // ShortRangeClass.cc:333-336 / DistDisp(slice, slice + skip, p1, p2): p1 = i, p2 = j
-      double raw[3], dA[3], dB[3];
-      displacement(pi, pj, sys, raw, dA);
-      double ra = sqrt(dA[0] * dA[0] + dA[1] * dA[1] + dA[2] * dA[2]);
-      SliceVal va = {0.0, 0.0}, vb = {0.0, 0.0};
-      if (live && (KIND != PA_TRICUBIC || DO_V)) va = slice_value<KIND, DO_V>(a.pa, tb, ra);
-      for (int l = l0; l < l0 + len; l += kStep) {
-        int listed = 0;
+      if (n == 0) continue;
+      // Few pairs: their walks are cut so that about two units come to a thread
+      int nsub = 1;
+      const int links = lend - lbeg;
+      if (KIND == PA_DAVID && a.bounds)
+        while (n * nsub < 2 * kThreads && 4 * nsub < links) nsub *= 2;
+      const int len = (links + nsub - 1) / nsub;
+      const int units = n * nsub;
+      for (int u0 = 0; u0 < units; u0 += kThreads) {
+        const int u = u0 + tid;
+        const int sub = u / n, e = u - sub * n;
+        int i, j;
+        bool live = u < units;
+        if (KIND == PA_DAVID && a.bounds) {
+          const int code = live ? s_list[e] : 0;
+          i = code >> 9;
+          j = code & 511;
+        } else {
+          i = e >> a.tile_log2;
+          j = e & (T - 1);
+          live = live && i < ni && j < nj && (ti != tj || j < i);
+        }
+        const int l0 = lbeg + sub * len, l1 = min(lend, l0 + len);
+        live = live && l0 < l1;
+        if (KIND != PA_TRICUBIC && !live) continue;  // the tricubic teams need whole warps
+        const size_t row = (size_t)a.skip * N * 3;
+        const double *pi = a.path + ((size_t)(a.slice1 + (live ? l0 : lbeg) * a.skip) * N + i0 + (live ? i : 0)) * 3;
+        const double *pj = a.path + ((size_t)(a.slice1 + (live ? l0 : lbeg) * a.skip) * N + j0 + (live ? j : 0)) * 3;
+        // ShortRangeClass.cc:333-336 / DistDisp(slice, slice + skip, p1, p2): p1 = i, p2 = j
+        double raw[3], dA[3], dB[3];
+        displacement(pi, pj, sys, raw, dA);
+        double ra = sqrt(dA[0] * dA[0] + dA[1] * dA[1] + dA[2] * dA[2]);
+        SliceVal va = {0.0, 0.0}, vb = {0.0, 0.0};
+        if (live && (KIND != PA_TRICUBIC || DO_V)) va = slice_value<KIND, DO_V>(a.pa, tb, ra);
+        for (int l = l0; l < l0 + len; l += kStep) {
+          int listed = 0;
 #pragma unroll 1
-        for (int k = 0; k < kStep; k++) {
-          bool in = false;
-          PathTerm tt;
-          if (live && l + k < l1) {
-          pi += row;
-          pj += row;
-          displacement(pi, pj, sys, raw, dB);
-          double rb = sqrt(dB[0] * dB[0] + dB[1] * dB[1] + dB[2] * dB[2]);
-          if (KIND != PA_TRICUBIC || DO_V) vb = slice_value<KIND, DO_V>(a.pa, tb, rb);
-          const double e0 = dA[0] - dB[0], e1 = dA[1] - dB[1], e2 = dA[2] - dB[2];
-          double s2 = e0 * e0 + e1 * e1 + e2 * e2;
-          double rl = rb, fl = vb.f;  // the link's second length and value
-          if (!(s2 < a.near2)) {      // the image at the second slice that follows the first (PathClass.h:720-735)
-            double dl[3];
+          for (int k = 0; k < kStep; k++) {
+            bool in = false;
+            PathTerm tt;
+            if (live && l + k < l1) {
+              pi += row;
+              pj += row;
+              displacement(pi, pj, sys, raw, dB);
+              double rb = sqrt(dB[0] * dB[0] + dB[1] * dB[1] + dB[2] * dB[2]);
+              if (KIND != PA_TRICUBIC || DO_V) vb = slice_value<KIND, DO_V>(a.pa, tb, rb);
+              const double e0 = dA[0] - dB[0], e1 = dA[1] - dB[1], e2 = dA[2] - dB[2];
+              double s2 = e0 * e0 + e1 * e1 + e2 * e2;
+              double rl = rb, fl = vb.f;  // the link's second length and value
+              if (!(s2 < a.near2)) {      // the image at the second slice that follows the first (PathClass.h:720-735)
+                double dl[3];
 #pragma unroll
-            for (int x = 0; x < 3; x++)
-              dl[x] = radd(raw[x], rmul(rint(rmul(rsub(dA[x], raw[x]), sys.boxinv[x])), sys.box[x]));
-            const double g0 = dA[0] - dl[0], g1 = dA[1] - dl[1], g2 = dA[2] - dl[2];
-            s2 = g0 * g0 + g1 * g1 + g2 * g2;
-            rl = sqrt(dl[0] * dl[0] + dl[1] * dl[1] + dl[2] * dl[2]);
-            if (KIND != PA_TRICUBIC || DO_V) fl = slice_value<KIND, false>(a.pa, tb, rl).f;
-          }
-          if (KIND == PA_DAVID) {
-            du += 0.5 * (va.f + fl);
-            const DDavid<double> &d = a.pa.d64;
-            if (d.num_terms > 0) {
-              const double q = 0.5 * (ra + rl);
-              if (s2 > 0.0 && q < d.grid.end) {
-                const size_t o = (size_t)(a.level + d.tau_pos) * d.grid.n * d.ncols;
-                du += david_offdiag_add<double>(d.grid, d.duy + o, d.dud2 + o, d.ncols, d.num_terms, 0.0, s2, q,
-                                                ra - rl);
+                for (int x = 0; x < 3; x++)
+                  dl[x] = radd(raw[x], rmul(rint(rmul(rsub(dA[x], raw[x]), sys.boxinv[x])), sys.box[x]));
+                const double g0 = dA[0] - dl[0], g1 = dA[1] - dl[1], g2 = dA[2] - dl[2];
+                s2 = g0 * g0 + g1 * g1 + g2 * g2;
+                rl = sqrt(dl[0] * dl[0] + dl[1] * dl[1] + dl[2] * dl[2]);
+                if (KIND != PA_TRICUBIC || DO_V) fl = slice_value<KIND, false>(a.pa, tb, rl).f;
               }
-            }
-          } else if (KIND == PA_COULOMB) {
-            du += a.pa.c64.z1z2 / (0.5 * (ra + rl)) - 0.5 * (va.f + fl);
-          } else {
-            const TriPrep<double> pr = tricubic_prep<double>(a.pa.t64, 0.5 * (ra + rl), ra - rl, s2);
-            in = pr.inside;
-            if (pr.inside) {
-              for (int x = 0; x < 3; x++) tt.u[x] = pr.u[x];
-              tt.cell = pr.cell;
-            } else if (DO_V) {
-              du += 0.5 * (va.f + fl);
-            } else {
-              du += 0.5 * (slice_value<KIND, false>(a.pa, tb, ra).f + slice_value<KIND, false>(a.pa, tb, rl).f);
-            }
-          }
-          if (DO_V) vs += (l + k == 0 ? 0.5 : 1.0) * va.v;
+              if (KIND == PA_DAVID) {
+                du += 0.5 * (va.f + fl);
+                const DDavid<double> &d = a.pa.d64;
+                if (d.num_terms > 0) {
+                  const double q = 0.5 * (ra + rl);
+                  if (s2 > 0.0 && q < d.grid.end) {
+                    const size_t o = (size_t)(a.level + d.tau_pos) * d.grid.n * d.ncols;
+                    du += david_offdiag_add<double>(d.grid, d.duy + o, d.dud2 + o, d.ncols, d.num_terms, 0.0, s2, q,
+                                                    ra - rl);
+                  }
+                }
+              } else if (KIND == PA_COULOMB) {
+                du += a.pa.c64.z1z2 / (0.5 * (ra + rl)) - 0.5 * (va.f + fl);
+              } else {
+                const TriPrep<double> pr = tricubic_prep<double>(a.pa.t64, 0.5 * (ra + rl), ra - rl, s2);
+                in = pr.inside;
+                if (pr.inside) {
+                  for (int x = 0; x < 3; x++) tt.u[x] = pr.u[x];
+                  tt.cell = pr.cell;
+                } else if (DO_V) {
+                  du += 0.5 * (va.f + fl);
+                } else {
+                  du += 0.5 * (slice_value<KIND, false>(a.pa, tb, ra).f + slice_value<KIND, false>(a.pa, tb, rl).f);
+                }
+              }
+              if (DO_V) vs += (l + k == 0 ? 0.5 : 1.0) * va.v;
 #pragma unroll
-          for (int x = 0; x < 3; x++) dA[x] = dB[x];
-          ra = rb;
-          va = vb;
+              for (int x = 0; x < 3; x++) dA[x] = dB[x];
+              ra = rb;
+              va = vb;
+            }
+            if (KIND == PA_TRICUBIC) {
+              const unsigned m = __ballot_sync(0xffffffffu, in);
+              if (in) E[listed + __popc(m & ((1u << lane) - 1u))] = tt;
+              listed += __popc(m);
+            }
           }
           if (KIND == PA_TRICUBIC) {
-            const unsigned m = __ballot_sync(0xffffffffu, in);
-            if (in) E[listed + __popc(m & ((1u << lane) - 1u))] = tt;
-            listed += __popc(m);
+            // The in-fit terms of the warp's step, gathered by teams of four
+            // lanes: a cell's node pair is one 128-byte line a team, against a line
+            // a lane.
+            __syncwarp();
+            for (int x = lane >> 2; x < listed; x += 8) du += team_part(tb.F, a.pa.t64, E[x], lane & 3);
+            __syncwarp();
           }
         }
-        if (KIND == PA_TRICUBIC) {
-          // The in-fit terms of the warp's step, gathered by teams of four
-          // lanes: a cell's node pair is one 128-byte line a team, against a line
-          // a lane.
-          __syncwarp();
-          for (int x = lane >> 2; x < listed; x += 8) du += team_part(tb.F, a.pa.t64, E[x], lane & 3);
-          __syncwarp();
-        }
+        if (DO_V && live && l1 == a.nlinks) vs += 0.5 * va.v;
       }
-      if (DO_V && live && l1 == a.nlinks) vs += 0.5 * va.v;
-    }
-    if (lists) n = 0;  // walked
+      if (lists) n = 0;  // walked
     }
   }
   // this block's sums, then the last block adds every block's in block order
