@@ -22,8 +22,8 @@
 //    evaluating warps' sums and, only before it commits, for the samplers
 //    (two named barriers, so a sampler may take longer than the terms); counters
 //    and records are the sampler warp's; per-level constants are formed once a
-//    job; quotients by an FP32 reciprocal; cells and images by magic-constant
-//    rounding on the FP64 pipe.  A stage of a 64-atom chain on 8 x 256 threads
+//    job; integer quotients by an FP32 reciprocal and a correction (div_fast,
+//    link_of); cells and images by magic-constant rounding on the FP64 pipe.  A stage of a 64-atom chain on 8 x 256 threads
 //    took 7100 cycles (terms 4000, then 3000 to the next stage) and takes 5900
 //    with the stamps it was measured by (terms 2900).
 //  * Gaussians come from a warp-parallel polar method that reproduces the
@@ -300,8 +300,8 @@ __device__ __forceinline__ double2 rho_new_k(double2 ro, const double *kv, const
 }
 
 // OLD and NEW action sums of one stage level over this CTA's share of the
-// (partner, link) items (the moved particle's kinetic links are summed by
-// the sampler warp, kinetic_sums).  Partner positions are read once and
+// (partner, link) items (the moved particle's kinetic links are summed apart,
+// kinetic_sums).  Partner positions are read once and
 // serve both copies.
 //  * R = double: the FP64 path; SHADOW adds the mixed-path sums alongside.
 //  * R = float, the mixed path: FP64 geometry, FP32 table arithmetic
@@ -597,9 +597,11 @@ __device__ __forceinline__ StageSums stage_sums(const BisectionArgs &a, const do
 
 // KineticClass::SingleAction (KineticClass.cc:33-90) of the moved particle's
 // links at one level, OLD and NEW, by one full warp (a link per lane, a
-// fixed shuffle tree), FP64 on both paths.  The sampler warp computes it
-// while the other warps evaluate the pair terms, so no evaluating thread
-// starts its partner loads late.  The sums are identical in every lane.
+// fixed shuffle tree), FP64 on both paths: the last evaluating warp behind its
+// pair terms, from four evaluating warps on, added to its own row of sh_red and
+// announced with it on ebar; with fewer the sampler, before it samples, in a row
+// of its own for which it arrives on ebar too (run_job's kinwarp).  The sums are
+// identical in every lane.
 __device__ __forceinline__ double2 kinetic_sums(const double (*w_old)[3], const double (*w_new)[3], int num_levels,
                                                 int lv, const DevSystem &sys, const LevelConst *lc, int lane) {
   double so = 0.0, sn = 0.0;
@@ -1256,11 +1258,12 @@ __device__ void run_job(const BisectionArgs &a, ChainState *cs, int window, unsi
           __syncwarp();
           Group::arrive(G.sbar, sthreads);
         }
-        // ---- reduce: warps -> CTA (warp 0) -> cluster (DSMEM, rank order) ----
+        // ---- reduce: warps -> CTA (warp 0) -> cluster (DSMEM) ----
         // The sums are bitwise the same in every CTA of the cluster, so every
         // CTA takes the same decision (and the same re-evaluation request).
         // Two values at a time, a warp's (then a rank's) partial a lane: values
-        // v and v + 1 in the warp's halves, added by a butterfly over 16 lanes.
+        // v and v + 1 in the warp's halves, added by a butterfly over 16 lanes, whose
+        // order is the same whichever partial came first.
         auto reduce = [&](double out[NV + 1]) {
           const int par = xc & 1;
           const int half = lane >> 4, w = lane & 15;
