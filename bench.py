@@ -889,9 +889,9 @@ def run_c5(args, P, timer, local, rank, agg, launches):
         ms, st = timer(P.lib().pimc_stream(d.h), lambda: moves_and_shift(d, bb, rounds), args.steps, args.warmup,
                        bb.stats)
         d.close()
-        # per round: the bisection launch, plus the neighbour-list kernels (bounds, fill, clear) with
-        # lists; per step the ShiftMove kernel
-        launches["n"] += args.steps * (rounds * (4 if skin > 0 else 1) + 1)
+        # per round: the bisection launch, plus the neighbour-list kernels (bounds, fill) with lists;
+        # per step the ShiftMove kernel
+        launches["n"] += args.steps * (rounds * (3 if skin > 0 else 1) + 1)
         ms, st = agg(ms, st)
         out = rates(ms, st)
         out["pair_evals_per_move"] = st["pair_evals"] / st["moves"]
