@@ -703,7 +703,7 @@ static int window_slots(const pimc_context *ctx, int num_levels) {
 // The rule is for one context that has the GPU.  Several contexts' chains at once,
 // a host thread each, thousands of moves a second in all, this rule against the
 // fixed shape of before (1 x 256 below 256 particles, else 8 x 256), L = 3:
-//   8 hardware queues (the driver's default), 8 / 16 / 64 contexts:
+//   8 hardware queues (CUDA's default), 8 / 16 / 64 contexts:
 //     N = 64: 1166 / 1147 / 1071 against 714 / 689 / 638;  N = 512: 347 / 459 / 545 against 428 / 427 / 420
 //   32 queues (CUDA_DEVICE_MAX_CONNECTIONS), 16 / 32 / 64 contexts:
 //     N = 64: 2083 / 1802 / 1710 against 1157 / 1119 / 934;  N = 128: 1906 / 966 / 1395 against 902 / 926 / 863

@@ -1,6 +1,7 @@
 """ShortRangeClass::d_dBeta and the energy terms of the pair walk (csrc/pair_path.cu) against the oracle, where
 its rules switch: particle tiles, link chunks, the cut at half a box between two slices, and the lists of pairs
-within a short table's range (taken from 256 particles on for tables that end below 0.3 box sides)."""
+within a short table's range (taken from 256 particles and 5e7 range / side (pair, link)s on for tables that end
+below 0.3 box sides)."""
 import math
 
 import numpy as np
